@@ -7,7 +7,8 @@
 //  * small fronts (N <= 160 f64 / 224 f32): one CTA assembles the front in
 //    shared memory (zero, scatter A entries, extend-add each child's update
 //    matrix in turn), runs the partial Cholesky of its ns pivot columns and
-//    writes the factor panel and the update matrix back;
+//    writes the factor panel, the update matrix and the inverses of the
+//    panel's diagonal blocks (front_small.cuh);
 //  * large fronts: entries are scattered into the (pre-zeroed) global front,
 //    children are extend-added one child slot per launch (so two children of
 //    a front never race), then every 64-column panel is factored by a panel
@@ -21,128 +22,23 @@
 // reports DCT_ERR_ZERO_PIVOT.  No device assert or trap is used.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "dct_internal.h"
 #include "factor_diag.cuh"
 #include "factor_lu.cuh"
+#include "front_small.cuh"
 #include "tile_mm.cuh"
 #include "tc_common.cuh"
 
 namespace dct {
 namespace {
 
-template <typename T>
-__device__ __forceinline__ T load_val(const void* p, int dtype, int64_t i) {
-  if constexpr (sizeof(T) == sizeof(cplx)) {
-    if (dtype == DCT_C128) return static_cast<const cplx*>(p)[i];
-  }
-  return dtype == DCT_F64 ? T(static_cast<const double*>(p)[i])
-                          : T(static_cast<const float*>(p)[i]);
-}
-
 // resident CTAs per SM the trailing-update kernel is compiled for: two for
 // real values, one for complex (its 4 x 4 accumulators and tile copies are
 // twice as wide)
 template <typename T>
 constexpr int kUpdMinBlocks = sizeof(T) > 8 ? 1 : 2;
-
-// ---------------------------------------------------------------- small
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-k_small_front(DevSym S, const PanelTask* __restrict__ tasks, const void* vals,
-              int vals_dtype, int64_t vals_stride, T* fronts,
-              int64_t front_stride, int* status) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* F = reinterpret_cast<T*>(smem_raw);
-  const int s = tasks[blockIdx.x].s;
-  const int b = blockIdx.y;
-  const int N = S.front_n[s];
-  const int ns = S.sn_first[s + 1] - S.sn_first[s];
-  const int tid = threadIdx.x;
-  T* out = fronts + int64_t(b) * front_stride + S.front_off[s];
-
-  for (int i = tid; i < N * N; i += blockDim.x) F[i] = T(0);
-  __syncthreads();
-  const int64_t a0 = S.amap_ptr[s], a1 = S.amap_ptr[s + 1];
-  for (int64_t q = a0 + tid; q < a1; q += blockDim.x)
-    F[S.amap_pos[q]] = load_val<T>(vals, vals_dtype,
-                                   int64_t(b) * vals_stride + S.amap_e[q]);
-  __syncthreads();
-  for (int ci = S.child_ptr[s]; ci < S.child_ptr[s + 1]; ++ci) {
-    const int c = S.child[ci];
-    const int nc = S.front_n[c];
-    const int nsc = S.sn_first[c + 1] - S.sn_first[c];
-    const int nbc = nc - nsc;
-    const T* U = fronts + int64_t(b) * front_stride + S.front_off[c];
-    const int32_t* rel = S.rel + S.rel_ptr[c];
-    for (int idx = tid; idx < nbc * nbc; idx += blockDim.x) {
-      const int i = idx % nbc, j = idx / nbc;
-      if (i >= j)
-        F[rel[i] + rel[j] * N] += U[(nsc + i) + int64_t(nsc + j) * nc];
-    }
-    __syncthreads();
-  }
-  // (1) the ns pivot columns: right-looking, updates confined to the panel
-  //     (rows below k, columns k+1 .. ns-1); each thread owns whole rows
-  for (int k = 0; k < ns; ++k) {
-    T piv = F[k + k * N];
-    const bool bad = !good_pivot(piv);
-    if (bad) piv = T(1);
-    const T d = sqrt(piv);
-    const T inv = T(1) / d;
-    for (int r = k + 1 + tid; r < N; r += blockDim.x) F[r + k * N] *= inv;
-    __syncthreads();
-    if (tid == 0) {
-      F[k + k * N] = d;
-      if (bad) flag_pivot(status, s, b);
-    }
-    for (int r = k + 1 + tid; r < N; r += blockDim.x) {
-      const T lrk = F[r + k * N];
-      const int cmax = min(r, ns - 1);
-      for (int c = k + 1; c <= cmax; ++c) F[r + c * N] -= lrk * F[c + k * N];
-    }
-    __syncthreads();
-  }
-  // (2) Schur complement of the boundary rows, F_BB -= L_B L_B^T, in 64 x 64
-  //     register tiles (4 x 4 per thread) of the lower triangle
-  const int nbr = N - ns;
-  const int jg = tid & 15, ag = tid >> 4;
-  for (int ti = 0; ti * 64 < nbr; ++ti)
-    for (int tj = 0; tj <= ti; ++tj) {
-      T acc[4][4];
-      zero_acc(acc);
-      int ra[4], rb[4];
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        ra[p] = min(ns + ti * 64 + ag + 16 * p, N - 1);
-        rb[p] = min(ns + tj * 64 + jg + 16 * p, N - 1);
-      }
-      for (int k = 0; k < ns; ++k) {
-        T x[4], y[4];
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          x[p] = F[ra[p] + k * N];
-          y[p] = F[rb[p] + k * N];
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) acc[p][q] += x[p] * y[q];
-      }
-#pragma unroll
-      for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int i = ti * 64 + ag + 16 * p, j = tj * 64 + jg + 16 * q;
-          if (i < nbr && j <= i) F[(ns + i) + (ns + j) * N] -= acc[p][q];
-        }
-    }
-  __syncthreads();
-  // the whole front, upper part as zeros, so the buffer needs no clearing
-  for (int i = tid; i < N * N; i += blockDim.x) {
-    const int r = i % N, c = i / N;
-    out[i] = r >= c ? F[i] : T(0);
-  }
-}
 
 // ------------------------------------------------------------ large: setup
 // general plans (fronts2 non-null): the transposed entries, through the
@@ -418,15 +314,14 @@ k_large_update(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
 }
 
 // task: s, p.  D_p^{-1} of the factored diagonal block of panel p of a small
-// front, written column-major (ld w) at dinv + dinv_off[s] + p*64*64.
-template <typename T>
+// general front, written column-major (ld w) at dinv + dinv_off[s] + p*64*64.
 __global__ void __launch_bounds__(kThreads)
-k_panel_inverse(DevSym S, const PanelTask* __restrict__ tasks, const T* fronts,
-                int64_t front_stride, T* dinv, const int64_t* dinv_off,
+k_panel_inverse(DevSym S, const PanelTask* __restrict__ tasks, const double* fronts,
+                int64_t front_stride, double* dinv, const int64_t* dinv_off,
                 int64_t dinv_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* L = reinterpret_cast<T*>(smem_raw);       // ld kDLD
-  T* X = L + kPanel * kDLD;                     // ld kDLD
+  double* L = reinterpret_cast<double*>(smem_raw);       // ld kDLD
+  double* X = L + kPanel * kDLD;                     // ld kDLD
   const PanelTask tk = tasks[blockIdx.x];
   const int b = blockIdx.y;
   const int s = tk.s;
@@ -434,10 +329,10 @@ k_panel_inverse(DevSym S, const PanelTask* __restrict__ tasks, const T* fronts,
   const int ns = S.sn_first[s + 1] - S.sn_first[s];
   const int c0 = tk.p * kPanel;
   const int w = min(kPanel, ns - c0);
-  const T* F = fronts + int64_t(b) * front_stride + S.front_off[s];
-  diag_load<T, kThreads>(F, N, c0, w, L, X);
-  diag_chol_inv<T, kThreads, false>(L, X, nullptr, s, b);
-  T* out = dinv + int64_t(b) * dinv_stride + dinv_off[s] + int64_t(tk.p) * kPanel * kPanel;
+  const double* F = fronts + int64_t(b) * front_stride + S.front_off[s];
+  diag_load<double, kThreads>(F, N, c0, w, L, X);
+  diag_chol_inv<double, kThreads, false>(L, X, nullptr, s, b);
+  double* out = dinv + int64_t(b) * dinv_stride + dinv_off[s] + int64_t(tk.p) * kPanel * kPanel;
   for (int idx = threadIdx.x; idx < w * w; idx += blockDim.x) {
     const int r = idx % w, c = idx / w;
     out[r + c * w] = X[r + c * kDLD];
@@ -611,20 +506,24 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
   const int nb = P->nbatch;
   cudaError_t e = cudaSuccess;
   const int small_max = P->tune.small_front_max;
-  const size_t small_smem = sizeof(T) * (size_t(small_max) * small_max + small_max);
+  const size_t lu_smem = sizeof(T) * (size_t(small_max) * small_max + small_max);
   const size_t panel_smem = sizeof(T) * (2 * kPanel * kPanel);
   // the update kernel's tiles, or factor_diag's D and X, whichever is larger
   constexpr int kUpdateElems =
       2 * kPanel * kUT > kDiagSmemElems ? 2 * kPanel * kUT : kDiagSmemElems;
   const size_t update_smem = sizeof(T) * kUpdateElems;
   // attributes are per device: set them on every call (cheap host calls)
-  e = cudaFuncSetAttribute(k_small_front<T>,
+  e = cudaFuncSetAttribute(k_small_front<T, kThreads>,
                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(small_smem));
+                           static_cast<int>(small_smem<T>(small_max)));
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_small_front<T, kThreads / 2>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(small_smem<T>(std::min(kSmallNarrow, small_max))));
   if constexpr (sizeof(T) == 8) {
     if (e == cudaSuccess && lu)
       e = cudaFuncSetAttribute(k_small_front_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(small_smem));
+                               static_cast<int>(lu_smem));
   }
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_large_panel<T>,
@@ -646,9 +545,9 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
     const PanelTask* t = tasks + L.first;
     switch (L.kind) {
       case kSmallFront: {
-        const size_t smem = sizeof(T) * (size_t(L.arg) * L.arg + L.arg);
         if constexpr (sizeof(T) == 8) {
           if (lu) {
+            const size_t smem = sizeof(T) * (size_t(L.arg) * L.arg + L.arg);
             k_small_front_lu<<<grid, kThreads, smem, st>>>(
                 P->ds, t, static_cast<const double*>(vals), vals_stride, P->d_tr,
                 reinterpret_cast<double*>(fronts), reinterpret_cast<double*>(fronts2),
@@ -656,9 +555,13 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
             break;
           }
         }
-        k_small_front<T><<<grid, kThreads, smem, st>>>(
-            P->ds, t, vals, vals_dtype, vals_stride, fronts, P->front_stride,
-            P->status);
+        const bool narrow = L.arg <= kSmallNarrow;
+        e = launch_pdl(narrow ? k_small_front<T, kThreads / 2> : k_small_front<T, kThreads>, grid,
+                       dim3(narrow ? kThreads / 2 : kThreads), small_smem<T>(L.arg), st, P->ds, t,
+                       vals, vals_dtype, vals_stride, fronts, P->front_stride,
+                       static_cast<T*>(P->dinv), static_cast<const int64_t*>(P->d_dinv_off),
+                       P->dinv_stride, P->status);
+        if (e != cudaSuccess) return e;
         break;
       }
       case kLargeScatter:
@@ -709,30 +612,28 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
     e = P->prof.end(st);
     if (e != cudaSuccess) return e;
   }
-  // inverses of the diagonal blocks of small fronts, for the substitution
-  // (large fronts store theirs while factoring)
-  const size_t inv_smem = sizeof(T) * kDiagSmemElems;
-  e = cudaFuncSetAttribute(k_panel_inverse<T>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(inv_smem));
-  if (e != cudaSuccess) return e;
-  const int64_t ninv = int64_t(P->inv.tasks.size());
-  if (ninv > 0) {
-    e = P->prof.begin(kPanelInverse, 0.0, 0.0, st);
-    if (e != cudaSuccess) return e;
-    k_panel_inverse<T><<<dim3(static_cast<unsigned>(ninv), nb), kThreads, inv_smem,
-                         st>>>(P->ds, P->inv.d_tasks, fronts, P->front_stride,
-                               static_cast<T*>(P->dinv), P->d_dinv_off,
-                               P->dinv_stride);
-    if (lu)
-      k_panel_inverse<T><<<dim3(static_cast<unsigned>(ninv), nb), kThreads, inv_smem,
-                           st>>>(P->ds, P->inv.d_tasks, fronts2, P->front_stride,
-                                 static_cast<T*>(P->dinv2), P->d_dinv_off,
-                                 P->dinv_stride);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    e = P->prof.end(st);
-    if (e != cudaSuccess) return e;
+  // general plans: inverses of the diagonal blocks of small fronts, for the
+  // substitution (the symmetric types' fronts, and large ones, store theirs
+  // while factoring)
+  if constexpr (sizeof(T) == 8) {
+    const int64_t ninv = int64_t(P->inv.tasks.size());
+    if (lu && ninv > 0) {
+      const size_t inv_smem = sizeof(T) * kDiagSmemElems;
+      e = cudaFuncSetAttribute(k_panel_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(inv_smem));
+      if (e == cudaSuccess) e = P->prof.begin(kPanelInverse, 0.0, 0.0, st);
+      if (e != cudaSuccess) return e;
+      const dim3 grid(static_cast<unsigned>(ninv), nb);
+      k_panel_inverse<<<grid, kThreads, inv_smem, st>>>(
+          P->ds, P->inv.d_tasks, fronts, P->front_stride, static_cast<double*>(P->dinv),
+          P->d_dinv_off, P->dinv_stride);
+      k_panel_inverse<<<grid, kThreads, inv_smem, st>>>(
+          P->ds, P->inv.d_tasks, fronts2, P->front_stride, static_cast<double*>(P->dinv2),
+          P->d_dinv_off, P->dinv_stride);
+      e = cudaGetLastError();
+      if (e == cudaSuccess) e = P->prof.end(st);
+      if (e != cudaSuccess) return e;
+    }
   }
   e = run_linv<T>(P, st, P->fronts, P->dinv, P->linv);
   if (e == cudaSuccess && lu) e = run_linv<T>(P, st, P->fronts2, P->dinv2, P->linv2);
