@@ -209,12 +209,16 @@ void account_solve(const dct::Symbolic& S, dct::Schedule* sc, double es) {
   sc->flops.assign(sc->launches.size(), 0.0);
   sc->bytes.assign(sc->launches.size(), 0.0);
   sc->bytes_rhs.assign(sc->launches.size(), 0.0);
+  sc->max_ns.assign(sc->launches.size(), 0);
+  sc->max_nb.assign(sc->launches.size(), 0);
   for (size_t li = 0; li < sc->launches.size(); ++li) {
     const Launch& l = sc->launches[li];
     double f = 0, bf = 0, br = 0;
     for (int64_t q = l.first; q < l.first + l.count; ++q) {
       const PanelTask& t = sc->tasks[q];
       const int s = t.s, N = S.front_n[s], ns = S.ns(s);
+      sc->max_ns[li] = std::max(sc->max_ns[li], ns);
+      sc->max_nb[li] = std::max(sc->max_nb[li], N - ns);
       const double nbd = N - ns;
       if (l.kind == dct::kFwdSmall || l.kind == dct::kBwdSmall) {
         f += double(ns) * ns + 2 * nbd * ns;

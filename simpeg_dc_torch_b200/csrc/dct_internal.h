@@ -199,6 +199,10 @@ struct Schedule {
   std::vector<double> flops;
   std::vector<double> bytes;
   std::vector<double> bytes_rhs;
+  // per launch of a solve schedule: the most columns and boundary rows of its
+  // supernodes (sizes the shared memory of the single-panel kernels)
+  std::vector<int32_t> max_ns;
+  std::vector<int32_t> max_nb;
 };
 
 // Optional per-launch event timing (dct_plan_profile).

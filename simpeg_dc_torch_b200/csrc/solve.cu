@@ -2,9 +2,9 @@
 // permuted order, on row-major (n, k) right-hand sides.
 //
 // Per tree level (forward bottom-up, backward top-down):
-//   supernodes of one panel (ns <= 64): one CTA per (supernode, system, 64
-//     right-hand sides) does the whole step with the stored panel inverse
-//     D^{-1} (k_fwd_small / k_bwd_small);
+//   supernodes of one panel (ns <= 64): one CTA per (supernode, system, up to
+//     64 right-hand sides) does the whole step with the stored panel inverse
+//     D^{-1} (solve_small.cuh);
 //   larger supernodes: products with the explicit supernode inverse
 //     L_ss^{-1} (formed after the factorization) and with the boundary block
 //     L_Bs, in 64-row tiles on CUDA cores (float64 plans: k_fwd_linv,
@@ -23,7 +23,10 @@
 // (whose right-hand side is consumed by then) before the backward pass.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "dct_internal.h"
+#include "solve_small.cuh"
 #include "tile_mm.cuh"
 
 namespace dct {
@@ -35,11 +38,6 @@ constexpr int kLD = kPanel;             // leading dimension of smem tiles
 template <typename T>
 __device__ __forceinline__ void atomic_sub(T* p, T v) {
   atomicAdd(p, -v);
-}
-
-// a finished refinement: the remaining correction launches do nothing
-__device__ __forceinline__ bool ir_skip(const int* skip) {
-  return skip != nullptr && *reinterpret_cast<const volatile int*>(skip) != 0;
 }
 
 // resident CTAs per SM the CUDA-core substitution kernels are compiled for:
@@ -74,82 +72,6 @@ __device__ __forceinline__ void load_rhs(T* S, const T* __restrict__ src, int k,
       v = src[row * k + j0 + j];
     }
     S[r * kLD + j] = v;
-  }
-}
-
-// D^{-1} of panel p (w x w, column-major, ld w) as S[c][r] = Dinv[r, c]
-// (transposed = false: forward product) or S[r][c] = Dinv[r, c] (true).
-template <typename T>
-__device__ __forceinline__ void load_dinv(T* S, const T* __restrict__ Di, int w,
-                                          bool transposed) {
-#pragma unroll
-  for (int idx = threadIdx.x; idx < kLD * kLD; idx += kThreads) {
-    const int r = idx % kLD, c = idx / kLD;
-    const T v = (r < w && c < w) ? Di[r + c * w] : T(0);
-    if (transposed) S[r * kLD1 + c] = v;
-    else S[c * kLD1 + r] = v;
-  }
-}
-
-// ------------------------------------------------------------ forward, small
-// one CTA: y = D^{-1} b (to B), then b[boundary rows] -= L_B y (atomics, A)
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kSolveMinBlocks<T>) k_fwd_small(SolveArgs<T> g) {
-  if (ir_skip(g.skip)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S1 = reinterpret_cast<T*>(smem_raw);
-  T* S2 = S1 + kLD1 * kLD;
-  T* Y = S2 + kLD * kLD;
-  // the right-hand-side chunks of a task are adjacent CTAs (its L block
-  // is then read from HBM once and from L2 by the other chunks)
-  const int s = g.tasks[blockIdx.x / g.nchunk].s;
-  const int b = blockIdx.y;
-  const int j0 = (blockIdx.x % g.nchunk) * kRC;
-  const int rc = min(kRC, g.k - j0);
-  const DevSym& S = g.S;
-  const int N = S.front_n[s], first = S.sn_first[s];
-  const int w = S.sn_first[s + 1] - first;
-  const T* F = g.fronts + int64_t(b) * g.front_stride + S.front_off[s];
-  T* A = g.A + int64_t(b) * g.n * g.k;
-  T* Bo = g.B + int64_t(b) * g.n * g.k;
-  const int jg = threadIdx.x & 15, ag = threadIdx.x >> 4;
-  load_dinv(S1, g.dinv + b * g.dinv_stride + g.dinv_off[s], w, false);
-  load_rhs(S2, A, g.k, j0, rc, w, nullptr, first);
-  __syncthreads();
-  T acc[4][4];
-  zero_acc(acc);
-  mm_tile(S1, S2, w, w, acc);
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ag + 16 * p, j = jg + 16 * q;
-      Y[r * kLD + j] = acc[p][q];
-      if (r < w && j < rc) Bo[int64_t(first + r) * g.k + j0 + j] = acc[p][q];
-    }
-  const int32_t* rows = S.rows + S.rows_ptr[s];
-  for (int r0 = w; r0 < N; r0 += kLD) {
-    const int nr = min(kLD, N - r0);
-    __syncthreads();
-#pragma unroll
-    for (int idx = threadIdx.x; idx < kLD * kLD; idx += kThreads) {
-      const int r = idx % kLD, c = idx / kLD;
-      S1[c * kLD1 + r] = (r < nr && c < w) ? F[(r0 + r) + int64_t(c) * N] : T(0);
-    }
-    __syncthreads();
-    zero_acc(acc);
-    mm_tile(S1, Y, w, nr, acc);
-#pragma unroll
-    for (int p = 0; p < 4; ++p) {
-      const int r = ag + 16 * p;
-      if (r >= nr) continue;
-      T* dst = A + int64_t(rows[r0 + r]) * g.k + j0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int j = jg + 16 * q;
-        if (j < rc) atomic_sub(dst + j, acc[p][q]);
-      }
-    }
   }
 }
 
@@ -310,53 +232,6 @@ __device__ void boundary_product(const T* F, int N, int ns, int c0, int w,
     __syncthreads();
     mm_tile(S1, S2, ni, w, acc);
   }
-}
-
-// ------------------------------------------------------------ backward, small
-// one CTA: y -= L_B^T x_B ; x = D^{-T} y (to A)
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kSolveMinBlocks<T>) k_bwd_small(SolveArgs<T> g) {
-  if (ir_skip(g.skip)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S1 = reinterpret_cast<T*>(smem_raw);
-  T* S2 = S1 + kLD1 * kLD;
-  T* Y = S2 + kLD * kLD;
-  // the right-hand-side chunks of a task are adjacent CTAs (its L block
-  // is then read from HBM once and from L2 by the other chunks)
-  const int s = g.tasks[blockIdx.x / g.nchunk].s;
-  const int b = blockIdx.y;
-  const int j0 = (blockIdx.x % g.nchunk) * kRC;
-  const int rc = min(kRC, g.k - j0);
-  const DevSym& S = g.S;
-  const int N = S.front_n[s], first = S.sn_first[s];
-  const int w = S.sn_first[s + 1] - first;
-  const T* F = g.fronts + int64_t(b) * g.front_stride + S.front_off[s];
-  T* A = g.A + int64_t(b) * g.n * g.k;
-  const T* Bo = g.B + int64_t(b) * g.n * g.k;
-  const int jg = threadIdx.x & 15, ag = threadIdx.x >> 4;
-  T acc[4][4];
-  zero_acc(acc);
-  boundary_product(F, N, w, 0, w, S.rows + S.rows_ptr[s], A, g.k, j0, rc, S1,
-                   S2, acc);
-  __syncthreads();
-  // Y = y - acc
-  load_rhs(Y, Bo, g.k, j0, rc, w, nullptr, first);
-  __syncthreads();
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) Y[(ag + 16 * p) * kLD + jg + 16 * q] -= acc[p][q];
-  load_dinv(S1, g.dinv + b * g.dinv_stride + g.dinv_off[s], w, true);
-  __syncthreads();
-  zero_acc(acc);
-  mm_tile(S1, Y, w, w, acc);
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ag + 16 * p, j = jg + 16 * q;
-      if (r < w && j < rc) A[int64_t(first + r) * g.k + j0 + j] = acc[p][q];
-    }
 }
 
 // ------------------------------------------------------------ backward gemm
@@ -628,6 +503,41 @@ __global__ void k_ir_decide(IrState* ir, int* status, unsigned long long* resid_
   }
 }
 
+// right-hand sides per CTA of the single-panel kernels: the fewest columns
+// that hold k, or chunks of 64; chunks of 32 where those would leave a fifth
+// of the last tiles empty
+int small_columns(int k) {
+  if (k <= 32) return k <= 8 ? 8 : (k <= 16 ? 16 : 32);
+  const int c64 = (k + 63) / 64 * 64, c32 = (k + 31) / 32 * 32;
+  return 5 * c32 <= 4 * c64 ? 32 : 64;
+}
+
+template <typename T, int NC>
+cudaError_t launch_small(bool forward, SolveArgs<T> g, const SmallShape& sh, int64_t count,
+                         int nbatch, cudaStream_t st) {
+  const size_t smem = SmallPlaces<T, NC>(sh.w, sh.nb).bytes(sh.nb);
+  auto fn = forward ? k_fwd_small<T, NC> : k_bwd_small<T, NC>;
+  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(smem));
+  if (e != cudaSuccess) return e;
+  g.nchunk = (g.k + NC - 1) / NC;
+  return launch_pdl(fn, dim3(static_cast<unsigned>(count * g.nchunk), nbatch), dim3(kThreads),
+                    smem, st, g, sh);
+}
+template <typename T>
+cudaError_t launch_small(bool forward, const SolveArgs<T>& g, SmallShape sh, int64_t count,
+                         int nbatch, cudaStream_t st) {
+  constexpr int V = 16 / sizeof(T);
+  sh.wide = g.k % V == 0 && (reinterpret_cast<uintptr_t>(g.A) & 15) == 0 &&
+            (reinterpret_cast<uintptr_t>(g.B) & 15) == 0;
+  switch (small_columns(g.k)) {
+    case 8: return launch_small<T, 8>(forward, g, sh, count, nbatch, st);
+    case 16: return launch_small<T, 16>(forward, g, sh, count, nbatch, st);
+    case 32: return launch_small<T, 32>(forward, g, sh, count, nbatch, st);
+    default: return launch_small<T, 64>(forward, g, sh, count, nbatch, st);
+  }
+}
+
 inline dim3 grid1d(int64_t total, int ny) {
   int64_t blocks = (total + kThreads - 1) / kThreads;
   blocks = blocks < 1 ? 1 : (blocks > 148 * 16 ? 148 * 16 : blocks);
@@ -640,17 +550,15 @@ template <typename T>
 cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
                        bool transposed = false) {
   const int nchunk = (k + kRC - 1) / kRC;
-  const size_t smem3 = sizeof(T) * (kLD1 * kLD + 2 * kLD * kLD);
+  const size_t smem2 = sizeof(T) * (kLD1 * kLD + kLD * kLD);
   cudaError_t e = cudaSuccess;
-  const void* kernels[] = {reinterpret_cast<const void*>(k_fwd_small<T>),
-                           reinterpret_cast<const void*>(k_fwd_bnd<T>),
+  const void* kernels[] = {reinterpret_cast<const void*>(k_fwd_bnd<T>),
                            reinterpret_cast<const void*>(k_fwd_linv<T>),
                            reinterpret_cast<const void*>(k_bwd_linv<T>),
-                           reinterpret_cast<const void*>(k_bwd_small<T>),
                            reinterpret_cast<const void*>(k_bwd_gemm<T>)};
   for (const void* kf : kernels) {
     e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem3));
+                             static_cast<int>(smem2));
     if (e != cudaSuccess) return e;
   }
   SolveArgs<T> g{P->ds, nullptr, static_cast<const T*>(P->fronts), P->front_stride,
@@ -692,12 +600,18 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
       g.tasks = sc->d_tasks + L.first;
       dim3 grid(static_cast<unsigned>(L.count * nchunk), P->nbatch);
       switch (L.kind) {
-        case kFwdSmall: k_fwd_small<T><<<grid, kThreads, smem3, st>>>(g); break;
-        case kFwdBnd: k_fwd_bnd<T><<<grid, kThreads, smem3, st>>>(g); break;
-        case kFwdLinv: k_fwd_linv<T><<<grid, kThreads, smem3, st>>>(g); break;
-        case kBwdLinv: k_bwd_linv<T><<<grid, kThreads, smem3, st>>>(g); break;
-        case kBwdSmall: k_bwd_small<T><<<grid, kThreads, smem3, st>>>(g); break;
-        case kBwdGemm: k_bwd_gemm<T><<<grid, kThreads, smem3, st>>>(g); break;
+        case kFwdSmall:
+        case kBwdSmall:
+          // every launch of a solve but the first follows one of its own
+          e = launch_small<T>(pass == 0, g, SmallShape{sc->max_ns[li], sc->max_nb[li],
+                                                       pass == 1 || li > 0, 0},
+                              L.count, P->nbatch, st);
+          if (e != cudaSuccess) return e;
+          break;
+        case kFwdBnd: k_fwd_bnd<T><<<grid, kThreads, smem2, st>>>(g); break;
+        case kFwdLinv: k_fwd_linv<T><<<grid, kThreads, smem2, st>>>(g); break;
+        case kBwdLinv: k_bwd_linv<T><<<grid, kThreads, smem2, st>>>(g); break;
+        case kBwdGemm: k_bwd_gemm<T><<<grid, kThreads, smem2, st>>>(g); break;
         case kFwdLinvTc:
         case kFwdBndTc:
         case kBwdGemmTc:
