@@ -82,7 +82,9 @@ int dct_symbolic_get_array(const dct_symbolic* sym, const char* name,
 
 /* Host-side copy of the launch schedule a plan of this dtype would run
  * (which: 0 factorization, 1 forward, 2 backward substitution, 3 panel
- * inverses, 4 supernode inverses), for
+ * inverses, 4 supernode inverses, 5 factorization with the trailing updates
+ * in blocks of four panels, as float64 and complex plans run it -- 0 gives
+ * their update after every panel), for
  * inspection and CPU-side replay in tests.  tasks: 4 int32 per task
  * (supernode, panel or K start, t0, t1 or K end); launches: 5 int64 per launch (kind, level,
  * first task, task count, arg).  With null outputs only the counts are set. */

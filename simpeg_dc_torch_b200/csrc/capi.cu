@@ -205,6 +205,14 @@ dct_tuning resolve_tuning(int dtype, const dct_tuning* in) {
 }
 
 
+// Panels per block of a plan's trailing update.  Float64 and complex plans
+// take blocks of kUpdateBlockWide panels whatever the tuning says (it tunes
+// the float32 blocks): a tile is then read and written once per 256 columns
+// instead of once per 64.
+int plan_update_block(int dtype, const dct_tuning& t) {
+  return dtype == DCT_F32 ? t.update_block : dct::kUpdateBlockWide;
+}
+
 void account_solve(const dct::Symbolic& S, dct::Schedule* sc, double es) {
   sc->flops.assign(sc->launches.size(), 0.0);
   sc->bytes.assign(sc->launches.size(), 0.0);
@@ -757,12 +765,13 @@ int dct_symbolic_get_array(const dct_symbolic* h, const char* name, void* dst,
 int dct_symbolic_get_schedule(const dct_symbolic* h, int32_t dtype, int32_t which,
                               int32_t* tasks, int64_t* ntasks, int64_t* launches,
                               int64_t* nlaunches) {
-  if (!h || !ntasks || !nlaunches || which < 0 || which > 4 || !valid_dtype(dtype))
+  if (!h || !ntasks || !nlaunches || which < 0 || which > 5 || !valid_dtype(dtype))
     return fail(DCT_ERR_ARG, "bad arguments");
   dct::Schedule f, fw, bw, iv;
   const dct_tuning tu = default_tuning(dtype);
   const int small_max = tu.small_front_max;
-  build_factor_schedule(h->sym, small_max, update_tile(dtype), tu.update_block,
+  build_factor_schedule(h->sym, small_max, update_tile(dtype),
+                        which == 5 ? plan_update_block(dtype, tu) : tu.update_block,
                         dtype == DCT_F32, &f);
   build_solve_schedules(h->sym, dtype, tu, &fw, &bw);
   std::vector<int64_t> off;
@@ -773,7 +782,7 @@ int dct_symbolic_get_schedule(const dct_symbolic* h, int32_t dtype, int32_t whic
   int64_t ltot = 0;
   build_linv_schedule(h->sym, dtype, &lv, &loff, &ltot);
   const dct::Schedule& sc =
-      which == 0 ? f : (which == 1 ? fw : (which == 2 ? bw : (which == 3 ? iv : lv)));
+      which == 0 || which == 5 ? f : (which == 1 ? fw : (which == 2 ? bw : (which == 3 ? iv : lv)));
   const int64_t nt = int64_t(sc.tasks.size()), nl = int64_t(sc.launches.size());
   if (tasks) {
     if (*ntasks < nt) return fail(DCT_ERR_ARG, "task buffer too small");
@@ -864,9 +873,9 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
     return bail(rc);
   P->tune = resolve_tuning(dtype, tuning);
   const int small_max = P->tune.small_front_max;
-  build_factor_schedule(S, small_max, update_tile(dtype), P->tune.update_block,
-                        dtype == DCT_F32, &P->fact);
-  P->update_bpan = P->tune.update_block;
+  P->update_bpan = plan_update_block(dtype, P->tune);
+  build_factor_schedule(S, small_max, update_tile(dtype), P->update_bpan, dtype == DCT_F32,
+                        &P->fact);
   {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess &&

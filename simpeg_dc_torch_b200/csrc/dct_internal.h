@@ -88,14 +88,17 @@ constexpr int kSmallFrontF64 = 160;
 constexpr int kSmallFrontF32 = 224;
 constexpr int kSmallFrontC128 = 112;
 constexpr int kThreads = 256;
-constexpr int kRhsChunk = 64;   // right-hand sides per CTA in the solves
 constexpr int kUpdateTile = 64;   // trailing-update tile (rows = cols)
-// float32 fronts group their panels in blocks of this many for the trailing
-// update (see update_range); float64 fronts update after every panel
+// fronts group their panels in blocks of this many for the trailing update
+// (see update_range)
 #ifndef DCT_UPDATE_BLOCK_PANELS
 #define DCT_UPDATE_BLOCK_PANELS 4
 #endif
 constexpr int kUpdateBlockPanels = DCT_UPDATE_BLOCK_PANELS;
+#ifndef DCT_UPDATE_BLOCK_WIDE
+#define DCT_UPDATE_BLOCK_WIDE 4
+#endif
+constexpr int kUpdateBlockWide = DCT_UPDATE_BLOCK_WIDE;   // float64 and complex fronts
 
 // Column ranges of the trailing update that follows panel p of a supernode
 // with ns columns (front order N) when the panels are grouped in blocks of

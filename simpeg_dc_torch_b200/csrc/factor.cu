@@ -29,16 +29,17 @@
 #include "factor_lu.cuh"
 #include "front_small.cuh"
 #include "tile_mm.cuh"
+#include "tile_pipe.cuh"
 #include "tc_common.cuh"
 
 namespace dct {
 namespace {
 
-// resident CTAs per SM the trailing-update kernel is compiled for: two for
-// real values, one for complex (its 4 x 4 accumulators and tile copies are
-// twice as wide)
+// resident CTAs per SM the trailing-update kernel is compiled for: three for
+// real values (two, with the output tile loaded before the products, measured
+// 7 % slower), one for complex (its 4 x 4 accumulators are twice as wide)
 template <typename T>
-constexpr int kUpdMinBlocks = sizeof(T) > 8 ? 1 : 2;
+constexpr int kUpdMinBlocks = sizeof(T) > 8 ? 1 : 3;
 
 // ------------------------------------------------------------ large: setup
 // general plans (fronts2 non-null): the transposed entries, through the
@@ -128,6 +129,7 @@ k_large_extend_add(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
 }
 
 // ------------------------------------------------------------ large: panels
+constexpr int kPanelLd = kPanel + 4;   // 4 modulo 8: see dmma.cuh
 // task: s, p, t0 >= 1: the 64-row tile t0-1 below panel p becomes
 // F_rows D_p^{-T}, using the inverse stored when the diagonal was factored.
 // Float32 plans (im.img non-null) also write the rows' split image
@@ -139,11 +141,9 @@ __global__ void __launch_bounds__(kThreads)
 k_large_panel(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
               int64_t front_stride, const T* dinv, const int64_t* dinv_off,
               int64_t dinv_stride, ImgArgs im) {
-  pdl_wait();   // launched with launch_pdl: the predecessor's writes first
-  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* S1 = reinterpret_cast<T*>(smem_raw);   // [q][c] = Dinv[c, q]
-  T* S2 = S1 + kPanel * kPanel;              // [q][r] = F[r, q]
+  T* S2 = S1 + kPanel * kPanelLd;           // [q][r] = F[r, q]
   const PanelTask tk = tasks[blockIdx.x];
   const int b = blockIdx.y;
   const int s = tk.s;
@@ -156,95 +156,63 @@ k_large_panel(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
                 int64_t(tk.p) * kPanel * kPanel;
   const int r0 = c0 + w + (tk.t0 - 1) * kPanel;
   const int nr = min(kPanel, N - r0);
-#pragma unroll
-  for (int idx = threadIdx.x; idx < kPanel * kPanel; idx += kThreads) {
-    const int a = idx % kPanel, q = idx / kPanel;
-    S1[idx] = (a < w && q < w) ? Di[a + q * w] : T(0);
-    S2[idx] = (a < nr && q < w) ? F[(r0 + a) + int64_t(c0 + q) * N] : T(0);
-  }
+  pdl_wait();   // launched with launch_pdl: the predecessor's writes first
+  pdl_trigger();
+  small_load_cols(S1, kPanelLd, Di, w, w, w);
+  small_load_cols(S2, kPanelLd, F + r0 + int64_t(c0) * N, N, nr, w);
+  small_commit();
+  small_wait<0>();
   __syncthreads();
-  T acc[4][4];
-  zero_acc(acc);
-  mm64<T, kPanel, kPanel>(S1, S2, w, w, acc);
-  const int jg = threadIdx.x & 15, ag = threadIdx.x >> 4;
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int c = ag + 16 * p;
-    if (c >= w) continue;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = jg + 16 * q;
-      if (r < nr) F[(r0 + r) + int64_t(c0 + c) * N] = acc[p][q];
-    }
-  }
+  SmallTile<T, kPanel> acc;
+  acc.zero();
+  acc.template mul<false>(S1, kPanelLd, S2, (w + 3) & ~3, w, nr);
+  float* img = nullptr;
+  int R0 = 0, G = 0;
   if constexpr (sizeof(T) == 4) {
     if (im.img != nullptr) {
-      float* img = im.img + int64_t(b) * im.stride + im.off[im.pan_first[s] + tk.p];
-      const int R0 = img_origin(tk.p, ns), G = img_groups(tk.p, ns, N);
-#pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        const int c = ag + 16 * p;
-        if (c >= w) continue;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int r = jg + 16 * q;
-          if (r >= nr) continue;
-          const int gr = r0 + r - R0;
-          const float v = float(acc[p][q]);
-          const uint32_t h = tf32_rna(v);
-          img[img_index(G, 0, c / kImgK, gr >> 3, c % kImgK, gr & 7)] = __uint_as_float(h);
-          img[img_index(G, 1, c / kImgK, gr >> 3, c % kImgK, gr & 7)] = v - __uint_as_float(h);
-        }
-      }
+      img = im.img + int64_t(b) * im.stride + im.off[im.pan_first[s] + tk.p];
+      R0 = img_origin(tk.p, ns);
+      G = img_groups(tk.p, ns, N);
     }
   }
+  acc.each(w, [&](int c, int r, T& x) {
+    if (c >= w || r >= nr) return;
+    F[(r0 + r) + int64_t(c0 + c) * N] = x;
+    if constexpr (sizeof(T) == 4) {
+      if (img == nullptr) return;
+      const int gr = r0 + r - R0;
+      const float v = float(x);
+      const uint32_t h = tf32_rna(v);
+      img[img_index(G, 0, c / kImgK, gr >> 3, c % kImgK, gr & 7)] = __uint_as_float(h);
+      img[img_index(G, 1, c / kImgK, gr >> 3, c % kImgK, gr & 7)] = v - __uint_as_float(h);
+    }
+  });
 }
 
 // task: s, p, t0 = i, t1 = j (i >= j): 64 x 64 tile of the trailing block
-// that starts after panel p, F_ij -= L_i L_j^T with K = w (4 x 4 outputs per
-// thread, rows on the fast thread index so the tile is written coalesced).
+// that starts after panel p, F_ij -= L_i L_j^T over the columns of
+// update_range.
 // The CTA of tile (0, 0) -- the next panel's diagonal block -- factors that
 // block after its own update (no other task of the launch touches it).
 // t0 = -1: factor the diagonal block of panel p itself (a front's first panel).
 constexpr int kUT = kUpdateTile;
 
-// One tile update F_out[i, j] -= Fa_i Fb_j^T (K = w): rows ri.. of Fa and
-// rj.. of Fb in the panel's columns, 4 x 4 outputs per thread.
+// One tile update F_out[i, j] -= Fa_i Fb_j^T over the columns ka .. base - 1:
+// rows rj.. of Fb and ri.. of Fa, entries on or below the diagonal.
 template <typename T>
-__device__ __forceinline__ void tile_update(const T* Fa, const T* Fb, T* Fo, int N, int c0,
-                                            int w, int ri, int rj, int ni, int nj, T* As,
-                                            T* Bs) {
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int idx = tid; idx < kPanel * kUT; idx += kThreads) {
-    const int r = idx % kUT, k = idx / kUT;
-    const bool kin = k < w;
-    As[idx] = (kin && r < ni) ? Fa[(ri + r) + int64_t(c0 + k) * N] : T(0);
-    Bs[idx] = (kin && r < nj) ? Fb[(rj + r) + int64_t(c0 + k) * N] : T(0);
-  }
-  __syncthreads();
-  T acc[4][4];
-  zero_acc(acc);
-  mm64<T, kUT, kUT>(Bs, As, w, nj, acc);    // acc[p][q]: col ag+16p, row jg+16q
-  const int jg = tid & 15, ag = tid >> 4;
-  // all loads first, then the stores: the loads cannot be hoisted over
-  // stores to the same buffer, so a fused read-modify-write loop would
-  // serialise one global round trip per element
-  T cur[4][4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int cc = ag + 16 * p, rr = jg + 16 * q;
-      cur[p][q] = (cc < nj && rr < ni) ? Fo[(ri + rr) + int64_t(rj + cc) * N] : T(0);
-    }
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int cc = ag + 16 * p, rr = jg + 16 * q;
-      if (cc < nj && rr < ni) Fo[(ri + rr) + int64_t(rj + cc) * N] = cur[p][q] - acc[p][q];
-    }
+__device__ __forceinline__ void tile_update(const T* Fa, const T* Fb, T* Fo, int N, int ka,
+                                            int base, int ri, int rj, int ni, int nj, T* ring) {
+  SmallTile<T, kUT> cur, acc;
+  acc.zero();
+  ColStream<T, kUT> a(Fb + rj + int64_t(ka) * N, N, nj), b(Fa + ri + int64_t(ka) * N, N, ni);
+  TilePipe<T, kUT, false>::run(ring, base - ka, nj, ni, acc, a, b);
+  cur.each(nj, [&](int c, int r, T& v) {
+    v = c < nj && r < ni && ri + r >= rj + c ? Fo[(ri + r) + int64_t(rj + c) * N] : T(0);
+  });
+  tile_subtract(cur, acc);
+  cur.each(nj, [&](int c, int r, T& v) {
+    if (c < nj && r < ni && ri + r >= rj + c) Fo[(ri + r) + int64_t(rj + c) * N] = v;
+  });
 }
 
 // General plans (fronts2 non-null, float64): two products per tile, the lower
@@ -254,12 +222,10 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads, kUpdMinBlocks<T>)
 k_large_update(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
                int64_t front_stride, T* dinv, const int64_t* dinv_off,
-               int64_t dinv_stride, int* status, T* fronts2, T* dinv2, double pivot_floor) {
-  pdl_wait();   // launched with launch_pdl: the predecessor's writes first
-  pdl_trigger();
+               int64_t dinv_stride, int bpan, int* status, T* fronts2, T* dinv2,
+               double pivot_floor) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* As = reinterpret_cast<T*>(smem_raw);   // [k][row of tile i], ld 64
-  T* Bs = As + kPanel * kUT;                // [k][row of tile j], ld 64
+  T* ring = reinterpret_cast<T*>(smem_raw);
   const PanelTask tk = tasks[blockIdx.x];
   const int b = blockIdx.y;
   const int s = tk.s;
@@ -278,6 +244,8 @@ k_large_update(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
       Dv2 = dinv2 + int64_t(b) * dinv_stride + dinv_off[s];
     }
   }
+  pdl_wait();   // launched with launch_pdl: the predecessor's writes first
+  pdl_trigger();
   // the diagonal block of panel q (Cholesky and inverse, or LU and both
   // inverses)
   auto diag = [&](int q) {
@@ -285,27 +253,28 @@ k_large_update(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
     if constexpr (sizeof(T) == 8) {
       if (F2 != nullptr) {
         lu_diag<kThreads>(reinterpret_cast<double*>(F), reinterpret_cast<double*>(F2), N, cq,
-                          wq, reinterpret_cast<double*>(As),
+                          wq, reinterpret_cast<double*>(ring),
                           reinterpret_cast<double*>(Dv + int64_t(q) * kPanel * kPanel),
                           reinterpret_cast<double*>(Dv2 + int64_t(q) * kPanel * kPanel),
                           status, s, b, pivot_floor);
         return;
       }
     }
-    factor_diag<T, kThreads>(F, N, cq, wq, As, Dv + int64_t(q) * kPanel * kPanel, status, s, b);
+    factor_block<T, kThreads>(F, N, cq, wq, ring, Dv + int64_t(q) * kPanel * kPanel, status, s,
+                              b);
   };
   if (tk.t0 < 0) {
     diag(tk.p);
     return;
   }
+  const UpdateRange R = update_range(tk.p, ns, N, bpan);
   const int ri = base + tk.t0 * kUT, rj = base + tk.t1 * kUT;
-  const int ni = min(kUT, N - ri), nj = min(kUT, N - rj);
+  const int ni = min(kUT, N - ri), nj = min(kUT, R.cend - rj);
   if (F2 == nullptr) {
-    tile_update<T>(F, F, F, N, c0, w, ri, rj, ni, nj, As, Bs);
+    tile_update<T>(F, F, F, N, R.ka, base, ri, rj, ni, nj, ring);
   } else {
-    tile_update<T>(F, F2, F, N, c0, w, ri, rj, ni, nj, As, Bs);
-    __syncthreads();   // the operand tiles are reloaded
-    tile_update<T>(F2, F, F2, N, c0, w, ri, rj, ni, nj, As, Bs);
+    tile_update<T>(F, F2, F, N, R.ka, base, ri, rj, ni, nj, ring);
+    tile_update<T>(F2, F, F2, N, R.ka, base, ri, rj, ni, nj, ring);
   }
   if (tk.t0 == 0 && tk.t1 == 0 && base < ns) {
     __syncthreads();   // this CTA's updates of the block are complete
@@ -507,10 +476,10 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
   cudaError_t e = cudaSuccess;
   const int small_max = P->tune.small_front_max;
   const size_t lu_smem = sizeof(T) * (size_t(small_max) * small_max + small_max);
-  const size_t panel_smem = sizeof(T) * (2 * kPanel * kPanel);
-  // the update kernel's tiles, or factor_diag's D and X, whichever is larger
-  constexpr int kUpdateElems =
-      2 * kPanel * kUT > kDiagSmemElems ? 2 * kPanel * kUT : kDiagSmemElems;
+  const size_t panel_smem = sizeof(T) * (2 * kPanel * kPanelLd);
+  // the update kernel's copy ring, or the diagonal block's workspace
+  constexpr int kDiagElems = kDiagSmemElems > kBlockElems<T> ? kDiagSmemElems : kBlockElems<T>;
+  constexpr int kUpdateElems = std::max(TilePipe<T, kUT, false>::kElems, kDiagElems);
   const size_t update_smem = sizeof(T) * kUpdateElems;
   // attributes are per device: set them on every call (cheap host calls)
   e = cudaFuncSetAttribute(k_small_front<T, kThreads>,
@@ -529,10 +498,11 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
     e = cudaFuncSetAttribute(k_large_panel<T>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              static_cast<int>(panel_smem));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_large_update<T>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(update_smem));
+  if constexpr (sizeof(T) != 4) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k_large_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(update_smem));
+  }
   if (e != cudaSuccess) return e;
   const PanelTask* tasks = P->fact.d_tasks;
   for (size_t li = 0; li < P->fact.launches.size(); ++li) {
@@ -599,8 +569,8 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
         } else {
           e = launch_pdl(k_large_update<T>, grid, dim3(kThreads), update_smem, st, P->ds, t,
                          fronts, P->front_stride, static_cast<T*>(P->dinv), P->d_dinv_off,
-                         P->dinv_stride, P->status, fronts2, static_cast<T*>(P->dinv2),
-                         P->pivot_floor);
+                         P->dinv_stride, P->update_bpan, P->status, fronts2,
+                         static_cast<T*>(P->dinv2), P->pivot_floor);
         }
         if (e != cudaSuccess) return e;
         break;

@@ -334,6 +334,13 @@ __device__ __forceinline__ int trapezoid_tiles(int nti, int ntj) {
   return ntj * (ntj + 1) / 2 + (nti - ntj) * ntj;
 }
 
+// the next tile of a phase, for a whole warp
+__device__ __forceinline__ int take_tile(int* next_tile) {
+  int q = 0;
+  if ((threadIdx.x & 31) == 0) q = atomicAdd(next_tile, 1);
+  return __shfl_sync(0xffffffffu, q, 0);
+}
+
 // X_ij of the panel inverse, 16 x 16 at (i16, j16), one warp; pend = end of
 // the panel's columns.  The sum is formed in the block's own place.
 template <typename T>
@@ -406,6 +413,86 @@ __device__ __forceinline__ void small_xblock(T* F, const T* xd, int ld, int i16,
       __syncwarp();
     }
   }
+}
+
+// The columns c0 .. pend (one panel) of the N x N block F: factored, the rows
+// below them solved, and their inverse but for its last row.  Every column
+// right of the panel still lacks the panel's update.  next_tile: a word of
+// shared memory, 0 when it returns.
+template <typename T, int NT>
+__device__ __forceinline__ void small_panel(T* F, T* xd, int ld, int N, int c0, int pend,
+                                            int* next_tile, int* status, int s, int b) {
+  constexpr int TS = kSyrkTile<T>, kW = NT / 32;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  for (int o = c0, blk = 0; o < pend; o += 16, ++blk) {
+    const int wb = min(16, pend - o), nx = o + wb;
+    // Columns o .. pend take the update of the block before.  Warp 0 does
+    // the tile of the next diagonal block and factors that at once; the
+    // others do the rest and the row of X that the block before completed.
+    const int nti = (N - o + TS - 1) / TS, ntj = (pend - o + TS - 1) / TS;
+    if (warp == 0) {
+      if (blk > 0) {
+        syrk_tile<16>(F, ld, N, o, o, pend, o - 16, 16);
+        __syncwarp();
+      }
+      small_leaf(F, xd, ld, o, wb, status, s, b);
+    } else if (warp < blk) {
+      small_xblock(F, xd, ld, o - 16, c0 + 16 * (warp - 1), pend);
+    }
+    if (blk > 0) {
+      const int nt = trapezoid_tiles(nti, ntj);
+      for (int q = take_tile(next_tile); q < nt; q = take_tile(next_tile)) {
+        int i, j;
+        trapezoid_tile(q, ntj, i, j);
+        syrk_tile<16>(F, ld, N, o + i * TS, o + j * TS, pend, o - 16, 16);
+      }
+    }
+    __syncthreads();
+    if (tid == 0) *next_tile = nx < pend ? 1 : 0;
+    if (warp == kW - 1)
+      small_leaf_inverse(F, xd, ld, o, wb);
+    else
+      for (int r = nx + tid; r < N; r += NT - 32) small_row_solve(F, xd, ld, o, wb, r);
+    __syncthreads();
+  }
+}
+// its last row, one warp per block (those of the first warps)
+template <typename T>
+__device__ __forceinline__ void small_panel_last(T* F, const T* xd, int ld, int c0, int pend) {
+  const int last = (pend - c0 + 15) / 16 - 1, warp = threadIdx.x >> 5;
+  if (warp < last) small_xblock(F, xd, ld, c0 + 16 * last, c0 + 16 * warp, pend);
+}
+
+// Shared memory (elements) of factor_block: 64 columns and what the loops
+// read past them
+template <typename T>
+constexpr int kBlockElems = small_ld<T>(kPanel) * kPanel + kPanel + 16;
+
+// The diagonal block of the panel at column c0 (width w) of a front in HBM (order
+// N): L is written back (lower part), D^{-1} (w x w, ld w) to inv.  sm:
+// kBlockElems elements.  The blocked steps above took the place of a 64 x 64
+// Cholesky with the inverse formed in three CTA-wide steps per 16 columns.
+template <typename T, int NT>
+__device__ __noinline__ void factor_block(T* Fg, int N, int c0, int w, T* sm, T* inv, int* status,
+                                          int s, int b) {
+  __shared__ int next_tile;
+  const int ld = small_ld<T>(kPanel);
+  T* xd = sm + ld * kPanel;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr int kW = NT / 32;
+  T* D = Fg + c0 + int64_t(c0) * N;
+  if (tid == 0) next_tile = 0;
+  for (int c = warp; c < w; c += kW)
+    for (int r = c + lane; r < w; r += 32) sm[r + c * ld] = D[r + int64_t(c) * N];
+  __syncthreads();
+  small_panel<T, NT>(sm, xd, ld, w, 0, w, &next_tile, status, s, b);
+  small_panel_last(sm, xd, ld, 0, w);
+  __syncthreads();
+  for (int c = warp; c < w; c += kW)
+    for (int r = lane; r < w; r += 32) {
+      if (r >= c) D[r + int64_t(c) * N] = sm[r + c * ld];
+      inv[r + c * w] = xinv(sm, xd, ld, r, c);
+    }
 }
 
 template <typename T, int NT>
@@ -504,50 +591,13 @@ k_small_front(DevSym S, const PanelTask* __restrict__ tasks, const void* vals, i
   __syncthreads();
 
   constexpr int TS = kSyrkTile<T>;
-  auto take = [&]() {   // the next tile of a phase, for a whole warp
-    int q = 0;
-    if (lane == 0) q = atomicAdd(&next_tile, 1);
-    return __shfl_sync(0xffffffffu, q, 0);
-  };
   for (int c0 = 0; c0 < ns; c0 += kPanel) {
     const int pend = min(c0 + kPanel, ns);
-    for (int o = c0, blk = 0; o < pend; o += 16, ++blk) {
-      const int wb = min(16, pend - o), nx = o + wb;
-      // Columns o .. pend take the update of the block before.  Warp 0 does
-      // the tile of the next diagonal block and factors that at once; the
-      // others do the rest and the row of X that the block before completed.
-      const int nti = (N - o + TS - 1) / TS, ntj = (pend - o + TS - 1) / TS;
-      if (warp == 0) {
-        if (blk > 0) {
-          syrk_tile<16>(F, ld, N, o, o, pend, o - 16, 16);
-          __syncwarp();
-        }
-        small_leaf(F, xd, ld, o, wb, status, s, b);
-      } else if (warp < blk) {
-        small_xblock(F, xd, ld, o - 16, c0 + 16 * (warp - 1), pend);
-      }
-      if (blk > 0) {
-        const int nt = trapezoid_tiles(nti, ntj);
-        for (int q = take(); q < nt; q = take()) {
-          int i, j;
-          trapezoid_tile(q, ntj, i, j);
-          syrk_tile<16>(F, ld, N, o + i * TS, o + j * TS, pend, o - 16, 16);
-        }
-      }
-      __syncthreads();
-      if (tid == 0) next_tile = nx < pend ? 1 : 0;
-      if (warp == kW - 1)
-        small_leaf_inverse(F, xd, ld, o, wb);
-      else
-        for (int r = nx + tid; r < N; r += NT - 32) small_row_solve(F, xd, ld, o, wb, r);
-      __syncthreads();
-    }
-    // the last row of X and the rest of the front
-    const int last = (pend - c0 + 15) / 16 - 1;
-    if (warp < last) small_xblock(F, xd, ld, c0 + 16 * last, c0 + 16 * warp, pend);
-    if (pend < N) {
+    small_panel<T, NT>(F, xd, ld, N, c0, pend, &next_tile, status, s, b);
+    small_panel_last(F, xd, ld, c0, pend);
+    if (pend < N) {   // the rest of the front
       const int nti = (N - pend + TS - 1) / TS, nt = trapezoid_tiles(nti, nti);
-      for (int q = take(); q < nt; q = take()) {
+      for (int q = take_tile(&next_tile); q < nt; q = take_tile(&next_tile)) {
         int i, j;
         trapezoid_tile(q, nti, i, j);
         syrk_tile<0>(F, ld, N, pend + i * TS, pend + j * TS, N, c0, pend - c0);

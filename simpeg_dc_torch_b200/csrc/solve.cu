@@ -7,9 +7,9 @@
 //     D^{-1} (solve_small.cuh);
 //   larger supernodes: products with the explicit supernode inverse
 //     L_ss^{-1} (formed after the factorization) and with the boundary block
-//     L_Bs, in 64-row tiles on CUDA cores (float64 plans: k_fwd_linv,
-//     k_fwd_bnd, k_bwd_gemm, k_bwd_linv) or in 128-row tiles on the tensor
-//     cores (float32 plans, solve_tc.cu).
+//     L_Bs, in 64-row tiles (float64 on the double tensor cores, complex on the
+//     FMA units: k_fwd_linv, k_fwd_bnd, k_bwd_gemm, k_bwd_linv) or in 128-row
+//     tiles (float32 plans, solve_tc.cu).
 //
 // Two work buffers A and B of nbatch*n*k elements are used so that no launch
 // ever reads a location that another CTA of the same launch writes:
@@ -27,253 +27,144 @@
 
 #include "dct_internal.h"
 #include "solve_small.cuh"
-#include "tile_mm.cuh"
+#include "tile_pipe.cuh"
 
 namespace dct {
 namespace {
 
-constexpr int kRC = kRhsChunk;          // right-hand sides per CTA (64)
-constexpr int kLD = kPanel;             // leading dimension of smem tiles
-
+// ------------------------------------------------------------ large supernodes
+// 64 rows of output x NC right-hand sides per CTA, K through the copy ring of
+// tile_pipe.cuh (float64 and complex plans; float32: solve_tc.cu).  V elements
+// of the right-hand sides are copied at a time: 16 bytes where their rows are
+// aligned, else one.
 template <typename T>
-__device__ __forceinline__ void atomic_sub(T* p, T v) {
-  atomicAdd(p, -v);
-}
+constexpr int kLargeCtas = sizeof(T) == 8 ? 3 : 1;
 
-// resident CTAs per SM the CUDA-core substitution kernels are compiled for:
-// their shared memory admits 4 (float) / 2 (double); 3 caps float at 85
-// registers
-template <typename T>
-constexpr int kSolveMinBlocks = sizeof(T) == 4 ? 3 : (sizeof(T) == 8 ? 2 : 1);
-
-// S1 (the "a" operand) uses a padded leading dimension: several loaders
-// store it transposed, which would otherwise hit one bank 32 times.
-constexpr int kLD1 = kLD + 1;
-
-template <typename T>
-__device__ __forceinline__ void mm_tile(const T* __restrict__ S1,
-                                        const T* __restrict__ S2, int K,
-                                        int arows, T (&acc)[4][4]) {
-  mm64<T, kLD1, kLD>(S1, S2, K, arows, acc);
-}
-
-// rows [r0, r0+nr) x right-hand sides [j0, j0+rc) of a (n, k) buffer into
-// S[r][j] (ld kLD), zero elsewhere; rows may be gathered through `map`.
-template <typename T>
-__device__ __forceinline__ void load_rhs(T* S, const T* __restrict__ src, int k,
-                                         int j0, int rc, int nr,
-                                         const int32_t* map, int64_t r0) {
-#pragma unroll
-  for (int idx = threadIdx.x; idx < kLD * kRC; idx += kThreads) {
-    const int r = idx / kRC, j = idx % kRC;
-    T v = T(0);
-    if (r < nr && j < rc) {
-      const int64_t row = map ? int64_t(map[r]) : r0 + r;
-      v = src[row * k + j0 + j];
-    }
-    S[r * kLD + j] = v;
-  }
-}
-
-// ------------------------------------------------------------ forward, boundary
-// large supernodes, after all of their panel steps: the 64-row tile t of the
-// boundary rows [ns, N) receives -L[tile, 0:ns] y_s (y_s = all panels, in B),
-// accumulated over the panels before one atomic update per element.
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kSolveMinBlocks<T>) k_fwd_bnd(SolveArgs<T> g) {
-  if (ir_skip(g.skip)) return;
+// y_s = L_ss^{-1} b_s, rows 64 t0 .. (B <- A rows)
+template <typename T, int NC, int V>
+__global__ void __launch_bounds__(kThreads, kLargeCtas<T>) k_fwd_linv(SolveArgs<T> g) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S1 = reinterpret_cast<T*>(smem_raw);
-  T* S2 = S1 + kLD1 * kLD;
   const PanelTask tk = g.tasks[blockIdx.x / g.nchunk];
   const int b = blockIdx.y;
-  const int j0 = (blockIdx.x % g.nchunk) * kRC;
-  const int rc = min(kRC, g.k - j0);
+  const int j0 = (blockIdx.x % g.nchunk) * NC;
+  const int rc = min(NC, g.k - j0);
+  const DevSym& S = g.S;
+  const int s = tk.s;
+  const int first = S.sn_first[s];
+  const int ns = S.sn_first[s + 1] - first;
+  const int r0 = tk.t0 * kPanel, nr = min(kPanel, ns - r0);
+  const T* X = g.linv + int64_t(b) * g.linv_stride + g.linv_off[s];
+  const T* A = g.A + int64_t(b) * g.n * g.k;
+  T* Bo = g.B + int64_t(b) * g.n * g.k;
+  pdl_wait();   // launched with launch_pdl: the predecessor's writes first
+  pdl_trigger();
+  SmallTile<T, NC> acc;
+  acc.zero();
+  ColStream<T, kPanel> a(X + r0, ns, nr);
+  RhsStream<T, NC, V, false> x(A, g.k, j0, rc, first, nullptr);
+  TilePipe<T, NC, false>::run(reinterpret_cast<T*>(smem_raw), r0 + nr, nr, rc, acc, a, x);
+  acc.each(nr, [&](int r, int j, T& v) {
+    if (r < nr && j < rc) Bo[int64_t(first + r0 + r) * g.k + j0 + j] = v;
+  });
+}
+
+// x_s = L_ss^{-T} y_s, rows 64 t0 .. (A <- B rows)
+template <typename T, int NC, int V>
+__global__ void __launch_bounds__(kThreads, kLargeCtas<T>) k_bwd_linv(SolveArgs<T> g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const PanelTask tk = g.tasks[blockIdx.x / g.nchunk];
+  const int b = blockIdx.y;
+  const int j0 = (blockIdx.x % g.nchunk) * NC;
+  const int rc = min(NC, g.k - j0);
+  const DevSym& S = g.S;
+  const int s = tk.s;
+  const int first = S.sn_first[s];
+  const int ns = S.sn_first[s + 1] - first;
+  const int r0 = tk.t0 * kPanel, nr = min(kPanel, ns - r0);
+  const T* X = g.linv + int64_t(b) * g.linv_stride + g.linv_off[s];
+  T* A = g.A + int64_t(b) * g.n * g.k;
+  const T* Bo = g.B + int64_t(b) * g.n * g.k;
+  pdl_wait();
+  pdl_trigger();
+  SmallTile<T, NC> acc;
+  acc.zero();
+  RowStream<T> a(X + r0 + int64_t(r0) * ns, ns, nr);
+  RhsStream<T, NC, V, false> x(Bo, g.k, j0, rc, first + r0, nullptr);
+  TilePipe<T, NC, true>::run(reinterpret_cast<T*>(smem_raw), ns - r0, nr, rc, acc, a, x);
+  acc.each(nr, [&](int r, int j, T& v) {
+    if (r < nr && j < rc) A[int64_t(first + r0 + r) * g.k + j0 + j] = v;
+  });
+}
+
+// the boundary rows ns + 64 t0 .. (in A) receive -L[rows, 0:ns] y_s, one atomic
+// update per element
+template <typename T, int NC, int V>
+__global__ void __launch_bounds__(kThreads, kLargeCtas<T>) k_fwd_bnd(SolveArgs<T> g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const PanelTask tk = g.tasks[blockIdx.x / g.nchunk];
+  const int b = blockIdx.y;
+  const int j0 = (blockIdx.x % g.nchunk) * NC;
+  const int rc = min(NC, g.k - j0);
   const DevSym& S = g.S;
   const int s = tk.s;
   const int N = S.front_n[s], first = S.sn_first[s];
   const int ns = S.sn_first[s + 1] - first;
-  const int r0 = ns + tk.t0 * kLD;
-  const int nr = min(kLD, N - r0);
+  const int r0 = ns + tk.t0 * kPanel, nr = min(kPanel, N - r0);
   const T* F = g.fronts + int64_t(b) * g.front_stride + S.front_off[s];
+  const int32_t* rows = S.rows + S.rows_ptr[s] + r0;
   T* A = g.A + int64_t(b) * g.n * g.k;
   const T* Bo = g.B + int64_t(b) * g.n * g.k;
-  const int jg = threadIdx.x & 15, ag = threadIdx.x >> 4;
-  T acc[4][4];
-  zero_acc(acc);
-  for (int c0 = 0; c0 < ns; c0 += kPanel) {
-    const int w = min(kPanel, ns - c0);
-    __syncthreads();
-#pragma unroll
-    for (int idx = threadIdx.x; idx < kLD * kLD; idx += kThreads) {
-      const int r = idx % kLD, c = idx / kLD;
-      S1[c * kLD1 + r] = (r < nr && c < w) ? F[(r0 + r) + int64_t(c0 + c) * N] : T(0);
-    }
-    load_rhs(S2, Bo, g.k, j0, rc, w, nullptr, first + c0);
-    __syncthreads();
-    mm_tile(S1, S2, w, nr, acc);
-  }
-  const int32_t* rows = S.rows + S.rows_ptr[s];
-#pragma unroll
-  for (int p = 0; p < 4; ++p) {
-    const int r = ag + 16 * p;
-    if (r >= nr) continue;
-    T* dst = A + int64_t(rows[r0 + r]) * g.k + j0;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int j = jg + 16 * q;
-      if (j < rc) atomic_sub(dst + j, acc[p][q]);
-    }
-  }
+  pdl_wait();
+  pdl_trigger();
+  SmallTile<T, NC> acc;
+  acc.zero();
+  ColStream<T, kPanel> a(F + r0, N, nr);
+  RhsStream<T, NC, V, false> x(Bo, g.k, j0, rc, first, nullptr);
+  TilePipe<T, NC, false>::run(reinterpret_cast<T*>(smem_raw), ns, nr, rc, acc, a, x);
+  acc.each(nr, [&](int r, int j, T& v) {
+    if (r < nr && j < rc) atomicAdd(A + int64_t(rows[r]) * g.k + j0 + j, -v);
+  });
 }
 
-// ------------------------------------------------------------ inverse products
-// large supernodes: y_s = L_ss^{-1} b_s, 64-row tile t0 per CTA (B <- A rows)
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kSolveMinBlocks<T>) k_fwd_linv(SolveArgs<T> g) {
-  if (ir_skip(g.skip)) return;
+// y_p (B) -= L[boundary rows, panel p]^T x[boundary rows]; a row list of at most
+// nrows rows (kGemmRows, or the launch's longest) is kept in shared memory
+constexpr int kGemmRows = 6144;
+template <typename T, int NC, int V>
+__global__ void __launch_bounds__(kThreads, kLargeCtas<T>)
+k_bwd_gemm(SolveArgs<T> g, int nrows) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S1 = reinterpret_cast<T*>(smem_raw);   // [k][a], ld kLD1: Linv[a, k]
-  T* S2 = S1 + kLD1 * kLD;                  // [k][j]: b[k, j]
+  T* ring = reinterpret_cast<T*>(smem_raw);
+  int32_t* rows_s = reinterpret_cast<int32_t*>(ring + TilePipe<T, NC, true>::kElems);
   const PanelTask tk = g.tasks[blockIdx.x / g.nchunk];
   const int b = blockIdx.y;
-  const int j0 = (blockIdx.x % g.nchunk) * kRC;
-  const int rc = min(kRC, g.k - j0);
-  const DevSym& S = g.S;
-  const int s = tk.s;
-  const int first = S.sn_first[s];
-  const int ns = S.sn_first[s + 1] - first;
-  const int r0 = tk.t0 * kLD, nr = min(kLD, ns - r0);
-  const T* X = g.linv + int64_t(b) * g.linv_stride + g.linv_off[s];
-  const T* A = g.A + int64_t(b) * g.n * g.k;
-  T* Bo = g.B + int64_t(b) * g.n * g.k;
-  T acc[4][4];
-  zero_acc(acc);
-  for (int k0 = 0; k0 <= r0; k0 += kLD) {
-    const int kw = min(kLD, ns - k0);
-    __syncthreads();
-#pragma unroll
-    for (int idx = threadIdx.x; idx < kLD * kLD; idx += kThreads) {
-      const int a = idx % kLD, kk = idx / kLD;
-      S1[kk * kLD1 + a] = (a < nr && kk < kw) ? X[(r0 + a) + int64_t(k0 + kk) * ns] : T(0);
-    }
-    load_rhs(S2, A, g.k, j0, rc, kw, nullptr, first + k0);
-    __syncthreads();
-    mm_tile(S1, S2, kw, nr, acc);
-  }
-  const int jg = threadIdx.x & 15, ag = threadIdx.x >> 4;
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ag + 16 * p, j = jg + 16 * q;
-      if (r < nr && j < rc) Bo[int64_t(first + r0 + r) * g.k + j0 + j] = acc[p][q];
-    }
-}
-
-// large supernodes: x_s = L_ss^{-T} y_s, 64-row tile t0 per CTA (A <- B rows)
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kSolveMinBlocks<T>) k_bwd_linv(SolveArgs<T> g) {
-  if (ir_skip(g.skip)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S1 = reinterpret_cast<T*>(smem_raw);   // [k][a], ld kLD1: Linv[k, a]
-  T* S2 = S1 + kLD1 * kLD;                  // [k][j]: y[k, j]
-  const PanelTask tk = g.tasks[blockIdx.x / g.nchunk];
-  const int b = blockIdx.y;
-  const int j0 = (blockIdx.x % g.nchunk) * kRC;
-  const int rc = min(kRC, g.k - j0);
-  const DevSym& S = g.S;
-  const int s = tk.s;
-  const int first = S.sn_first[s];
-  const int ns = S.sn_first[s + 1] - first;
-  const int r0 = tk.t0 * kLD, nr = min(kLD, ns - r0);
-  const T* X = g.linv + int64_t(b) * g.linv_stride + g.linv_off[s];
-  T* A = g.A + int64_t(b) * g.n * g.k;
-  const T* Bo = g.B + int64_t(b) * g.n * g.k;
-  T acc[4][4];
-  zero_acc(acc);
-  for (int k0 = r0; k0 < ns; k0 += kLD) {
-    const int kw = min(kLD, ns - k0);
-    __syncthreads();
-#pragma unroll
-    for (int idx = threadIdx.x; idx < kLD * kLD; idx += kThreads) {
-      const int kk = idx % kLD, a = idx / kLD;
-      S1[kk * kLD1 + a] = (a < nr && kk < kw) ? X[(k0 + kk) + int64_t(r0 + a) * ns] : T(0);
-    }
-    load_rhs(S2, Bo, g.k, j0, rc, kw, nullptr, first + k0);
-    __syncthreads();
-    mm_tile(S1, S2, kw, nr, acc);
-  }
-  const int jg = threadIdx.x & 15, ag = threadIdx.x >> 4;
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int r = ag + 16 * p, j = jg + 16 * q;
-      if (r < nr && j < rc) A[int64_t(first + r0 + r) * g.k + j0 + j] = acc[p][q];
-    }
-}
-
-// acc[c][j] += sum_r L[rows_r, c0 + c] x[rows_r, j] over the boundary rows
-// [ns, N) of front s (x gathered from A through the front's row list).
-template <typename T>
-__device__ void boundary_product(const T* F, int N, int ns, int c0, int w,
-                                 const int32_t* rows, const T* A, int k, int j0,
-                                 int rc, T* S1, T* S2, T (&acc)[4][4]) {
-  for (int i0 = ns; i0 < N; i0 += kLD) {
-    const int ni = min(kLD, N - i0);
-    __syncthreads();
-#pragma unroll
-    for (int idx = threadIdx.x; idx < kLD * kLD; idx += kThreads) {
-      const int r = idx % kLD, c = idx / kLD;
-      S1[r * kLD1 + c] = (r < ni && c < w) ? F[(i0 + r) + int64_t(c0 + c) * N] : T(0);
-    }
-    load_rhs(S2, A, k, j0, rc, ni, rows + i0, 0);
-    __syncthreads();
-    mm_tile(S1, S2, ni, w, acc);
-  }
-}
-
-// ------------------------------------------------------------ backward gemm
-// large supernodes: y_p (B) -= L[boundary rows, panel p]^T x[boundary rows]
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kSolveMinBlocks<T>) k_bwd_gemm(SolveArgs<T> g) {
-  if (ir_skip(g.skip)) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  T* S1 = reinterpret_cast<T*>(smem_raw);
-  T* S2 = S1 + kLD1 * kLD;
-  const PanelTask tk = g.tasks[blockIdx.x / g.nchunk];
-  const int b = blockIdx.y;
-  const int j0 = (blockIdx.x % g.nchunk) * kRC;
-  const int rc = min(kRC, g.k - j0);
+  const int j0 = (blockIdx.x % g.nchunk) * NC;
+  const int rc = min(NC, g.k - j0);
   const DevSym& S = g.S;
   const int s = tk.s;
   const int N = S.front_n[s], first = S.sn_first[s];
   const int ns = S.sn_first[s + 1] - first;
   const int c0 = tk.p * kPanel, w = min(kPanel, ns - c0);
   const T* F = g.fronts + int64_t(b) * g.front_stride + S.front_off[s];
+  const int32_t* rows = S.rows + S.rows_ptr[s] + ns;
   const T* A = g.A + int64_t(b) * g.n * g.k;
   T* Bo = g.B + int64_t(b) * g.n * g.k;
-  const int jg = threadIdx.x & 15, ag = threadIdx.x >> 4;
-  T acc[4][4];
-  zero_acc(acc);
-  boundary_product(F, N, ns, c0, w, S.rows + S.rows_ptr[s], A, g.k, j0, rc, S1,
-                   S2, acc);
-  T cur[4][4];
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = ag + 16 * p, j = jg + 16 * q;
-      cur[p][q] = (c < w && j < rc) ? Bo[int64_t(first + c0 + c) * g.k + j0 + j] : T(0);
-    }
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = ag + 16 * p, j = jg + 16 * q;
-      if (c < w && j < rc) Bo[int64_t(first + c0 + c) * g.k + j0 + j] = cur[p][q] - acc[p][q];
-    }
+  if (N - ns <= nrows)
+    for (int i = threadIdx.x; i < N - ns; i += kThreads) rows_s[i] = rows[i];
+  __syncthreads();
+  pdl_wait();
+  pdl_trigger();
+  SmallTile<T, NC> y, acc;
+  y.each(w, [&](int c, int j, T& v) {
+    v = c < w && j < rc ? Bo[int64_t(first + c0 + c) * g.k + j0 + j] : T(0);
+  });
+  acc.zero();
+  RowStream<T> a(F + ns + int64_t(c0) * N, N, w);
+  RhsStream<T, NC, V, true> x(A, g.k, j0, rc, 0, N - ns <= nrows ? rows_s : rows);
+  TilePipe<T, NC, true>::run(ring, N - ns, w, rc, acc, a, x);
+  tile_subtract(y, acc);
+  y.each(w, [&](int c, int j, T& v) {
+    if (c < w && j < rc) Bo[int64_t(first + c0 + c) * g.k + j0 + j] = v;
+  });
 }
 
 // ------------------------------------------------------------ permutations
@@ -503,38 +394,52 @@ __global__ void k_ir_decide(IrState* ir, int* status, unsigned long long* resid_
   }
 }
 
-// right-hand sides per CTA of the single-panel kernels: the fewest columns
-// that hold k, or chunks of 64; chunks of 32 where those would leave a fifth
-// of the last tiles empty
-int small_columns(int k) {
-  if (k <= 32) return k <= 8 ? 8 : (k <= 16 ? 16 : 32);
-  const int c64 = (k + 63) / 64 * 64, c32 = (k + 31) / 32 * 32;
-  return 5 * c32 <= 4 * c64 ? 32 : 64;
-}
+// right-hand sides per CTA of the kernels above: the fewest columns that hold
+// k, or chunks of 64 (whose fragments beyond k the double products skip)
+int tile_columns(int k) { return k <= 8 ? 8 : (k <= 16 ? 16 : (k <= 32 ? 32 : 64)); }
 
+// one launch of a substitution kind on tiles of NC right-hand sides
 template <typename T, int NC>
-cudaError_t launch_small(bool forward, SolveArgs<T> g, const SmallShape& sh, int64_t count,
-                         int nbatch, cudaStream_t st) {
-  const size_t smem = SmallPlaces<T, NC>(sh.w, sh.nb).bytes(sh.nb);
-  auto fn = forward ? k_fwd_small<T, NC> : k_bwd_small<T, NC>;
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-  if (e != cudaSuccess) return e;
+cudaError_t launch_tiles(int kind, SolveArgs<T> g, const SmallShape& sh, int64_t count, int nbatch,
+                         cudaStream_t st) {
   g.nchunk = (g.k + NC - 1) / NC;
-  return launch_pdl(fn, dim3(static_cast<unsigned>(count * g.nchunk), nbatch), dim3(kThreads),
-                    smem, st, g, sh);
+  const dim3 grid(static_cast<unsigned>(count * g.nchunk), nbatch), block(kThreads);
+  auto go = [&](auto fn, size_t smem, auto... more) {
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    return e != cudaSuccess ? e : launch_pdl(fn, grid, block, smem, st, g, more...);
+  };
+  if (kind == kFwdSmall || kind == kBwdSmall) {
+    const size_t smem = SmallPlaces<T, NC>(sh.w, sh.nb).bytes(sh.nb);
+    return kind == kFwdSmall ? go(k_fwd_small<T, NC>, smem, sh) : go(k_bwd_small<T, NC>, smem, sh);
+  }
+  if constexpr (sizeof(T) != 4) {
+    constexpr size_t km = sizeof(T) * TilePipe<T, NC, false>::kElems;
+    constexpr size_t mk = sizeof(T) * TilePipe<T, NC, true>::kElems;
+    const int nrows = std::min(sh.nb, kGemmRows);
+    constexpr int V = 16 / sizeof(T);
+    const bool wide = sh.wide != 0;
+    switch (kind) {
+      case kFwdLinv: return go(wide ? k_fwd_linv<T, NC, V> : k_fwd_linv<T, NC, 1>, km);
+      case kFwdBnd: return go(wide ? k_fwd_bnd<T, NC, V> : k_fwd_bnd<T, NC, 1>, km);
+      case kBwdLinv: return go(wide ? k_bwd_linv<T, NC, V> : k_bwd_linv<T, NC, 1>, mk);
+      case kBwdGemm:
+        return go(wide ? k_bwd_gemm<T, NC, V> : k_bwd_gemm<T, NC, 1>, mk + 4 * size_t(nrows), nrows);
+    }
+  }
+  return cudaErrorInvalidValue;
 }
 template <typename T>
-cudaError_t launch_small(bool forward, const SolveArgs<T>& g, SmallShape sh, int64_t count,
-                         int nbatch, cudaStream_t st) {
+cudaError_t launch_tiles(int kind, const SolveArgs<T>& g, SmallShape sh, int64_t count, int nbatch,
+                         cudaStream_t st) {
   constexpr int V = 16 / sizeof(T);
   sh.wide = g.k % V == 0 && (reinterpret_cast<uintptr_t>(g.A) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(g.B) & 15) == 0;
-  switch (small_columns(g.k)) {
-    case 8: return launch_small<T, 8>(forward, g, sh, count, nbatch, st);
-    case 16: return launch_small<T, 16>(forward, g, sh, count, nbatch, st);
-    case 32: return launch_small<T, 32>(forward, g, sh, count, nbatch, st);
-    default: return launch_small<T, 64>(forward, g, sh, count, nbatch, st);
+  switch (tile_columns(g.k)) {
+    case 8: return launch_tiles<T, 8>(kind, g, sh, count, nbatch, st);
+    case 16: return launch_tiles<T, 16>(kind, g, sh, count, nbatch, st);
+    case 32: return launch_tiles<T, 32>(kind, g, sh, count, nbatch, st);
+    default: return launch_tiles<T, 64>(kind, g, sh, count, nbatch, st);
   }
 }
 
@@ -549,21 +454,10 @@ inline dim3 grid1d(int64_t total, int ny) {
 template <typename T>
 cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
                        bool transposed = false) {
-  const int nchunk = (k + kRC - 1) / kRC;
-  const size_t smem2 = sizeof(T) * (kLD1 * kLD + kLD * kLD);
   cudaError_t e = cudaSuccess;
-  const void* kernels[] = {reinterpret_cast<const void*>(k_fwd_bnd<T>),
-                           reinterpret_cast<const void*>(k_fwd_linv<T>),
-                           reinterpret_cast<const void*>(k_bwd_linv<T>),
-                           reinterpret_cast<const void*>(k_bwd_gemm<T>)};
-  for (const void* kf : kernels) {
-    e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem2));
-    if (e != cudaSuccess) return e;
-  }
   SolveArgs<T> g{P->ds, nullptr, static_cast<const T*>(P->fronts), P->front_stride,
                  static_cast<const T*>(P->dinv), P->d_dinv_off, P->dinv_stride,
-                 bufA, bufB, P->sym.n, k, nchunk, P->status,
+                 bufA, bufB, P->sym.n, k, 1, P->status,
                  static_cast<const T*>(P->linv), P->d_linv_off, P->linv_stride,
                  P->dtype == DCT_F32 && P->ir != nullptr ? &P->ir->done : nullptr};
   constexpr bool kTc = sizeof(T) == 4;
@@ -598,20 +492,7 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
           cudaSuccess)
         return e;
       g.tasks = sc->d_tasks + L.first;
-      dim3 grid(static_cast<unsigned>(L.count * nchunk), P->nbatch);
       switch (L.kind) {
-        case kFwdSmall:
-        case kBwdSmall:
-          // every launch of a solve but the first follows one of its own
-          e = launch_small<T>(pass == 0, g, SmallShape{sc->max_ns[li], sc->max_nb[li],
-                                                       pass == 1 || li > 0, 0},
-                              L.count, P->nbatch, st);
-          if (e != cudaSuccess) return e;
-          break;
-        case kFwdBnd: k_fwd_bnd<T><<<grid, kThreads, smem2, st>>>(g); break;
-        case kFwdLinv: k_fwd_linv<T><<<grid, kThreads, smem2, st>>>(g); break;
-        case kBwdLinv: k_bwd_linv<T><<<grid, kThreads, smem2, st>>>(g); break;
-        case kBwdGemm: k_bwd_gemm<T><<<grid, kThreads, smem2, st>>>(g); break;
         case kFwdLinvTc:
         case kFwdBndTc:
         case kBwdGemmTc:
@@ -622,7 +503,12 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
             break;
           }
           return cudaErrorInvalidValue;
-        default: return cudaErrorInvalidValue;
+        default:
+          // every launch of a solve but the first follows one of its own
+          e = launch_tiles<T>(L.kind, g, SmallShape{sc->max_ns[li], sc->max_nb[li],
+                                                    pass == 1 || li > 0, 0},
+                              L.count, P->nbatch, st);
+          if (e != cudaSuccess) return e;
       }
       if ((e = cudaGetLastError()) != cudaSuccess) return e;
       if ((e = P->prof.end(st)) != cudaSuccess) return e;

@@ -49,10 +49,12 @@ __device__ __forceinline__ bool is_zero(const cplx& v) {
 
 // 64 x NC output tile of a CTA of 256 threads.  mul adds A B over K columns
 // (a multiple of 4), A read as [k][m] or (MK) [m][k], leading dimension la,
-// B as [k][n], leading dimension NC + 4; each(rows, f) visits this thread's
-// entries f(row, column, value) of the first `rows` rows, rounded up.
+// B as [k][n], leading dimension NC + 4; only the first `rows` rows and
+// `cols` columns of the tile need be right.  each(rows, f) visits this
+// thread's entries f(row, column, value) of the first `rows` rows, rounded up.
 template <typename T, int NC>
 struct SmallTile {
+  using Elem = T;
   static constexpr int JG = NC >= 16 ? 16 : 8, AG = kThreads / JG, P = 64 / AG, Q = NC / JG;
   T a[P][Q];
   __device__ __forceinline__ void zero() {
@@ -80,7 +82,7 @@ struct SmallTile {
     }
   }
   template <bool MK>
-  __device__ __forceinline__ void mul(const T* A, int la, const T* B, int K, int rows) {
+  __device__ __forceinline__ void mul(const T* A, int la, const T* B, int K, int rows, int) {
     const int np = (rows + AG - 1) / AG;
     if (np >= P) return mul_np<MK, P>(A, la, B, K);
     if constexpr (P > 1)
@@ -105,6 +107,7 @@ struct SmallTile {
 // warps in turn, so that a supernode of few rows still occupies all of them
 template <int NC>
 struct SmallTile<double, NC> {
+  using Elem = double;
   static constexpr int WM = NC == 64 ? 2 : (NC == 32 ? 4 : 8), WN = 8 / WM;
   static constexpr int MF = 8 / WM, NF = NC / 8 / WN, AG = 8;
   double a[MF][NF][2];
@@ -136,10 +139,11 @@ struct SmallTile<double, NC> {
     }
   }
   template <bool MK>
-  __device__ __forceinline__ void mul(const double* A, int la, const double* B, int K, int rows) {
-    const int nfr = (rows + 7) / 8 - (threadIdx.x >> 5) % WM;
+  __device__ __forceinline__ void mul(const double* A, int la, const double* B, int K, int rows,
+                                      int cols) {
+    const int warp = threadIdx.x >> 5, nfr = (rows + 7) / 8 - warp % WM;
     const int np = (nfr + WM - 1) / WM;
-    if (nfr <= 0) return;
+    if (nfr <= 0 || 8 * NF * (warp / WM) >= cols) return;
     if (np >= MF) return mul_np<MK, MF>(A, la, B, K);
     if constexpr (MF > 1)
       if (np == 1) return mul_np<MK, 1>(A, la, B, K);
@@ -311,7 +315,7 @@ k_fwd_small(SolveArgs<T> g, SmallShape sh) {
   small_commit();
   SmallTile<T, NC> acc;
   acc.zero();
-  acc.template mul<false>(Dv, at.ldd, Bt, w4, w);
+  acc.template mul<false>(Dv, at.ldd, Bt, w4, w, rc);
   __syncthreads();   // b is read: y takes its place
   acc.each(w, [&](int r, int j, T& v) {
     if (r < w) {
@@ -332,7 +336,7 @@ k_fwd_small(SolveArgs<T> g, SmallShape sh) {
     small_wait<0>();
     __syncthreads();
     acc.zero();
-    acc.template mul<false>(Lt, at.ldl, Bt, w4, nr);
+    acc.template mul<false>(Lt, at.ldl, Bt, w4, nr, rc);
     const int32_t* rs = rows_s + (r0 - w) % kSmallRows;
     acc.each(nr, [&](int r, int j, T& v) {
       if (r < nr && j < rc) atomicAdd(A + int64_t(rs[r]) * g.k + j0 + j, -v);
@@ -398,7 +402,7 @@ k_bwd_small(SolveArgs<T> g, SmallShape sh) {
     small_commit();
     small_wait<0>();
     __syncthreads();
-    acc.template mul<true>(Lt, at.ldl, Bt, (nr + 3) & ~3, w);
+    acc.template mul<true>(Lt, at.ldl, Bt, (nr + 3) & ~3, w, rc);
   }
   if (N == w && !sh.early) factors();
   small_commit();
@@ -416,7 +420,7 @@ k_bwd_small(SolveArgs<T> g, SmallShape sh) {
   });
   __syncthreads();
   acc.zero();
-  acc.template mul<true>(Dv, at.ldd, Bt, w4, w);
+  acc.template mul<true>(Dv, at.ldd, Bt, w4, w, rc);
   acc.each(w, [&](int r, int j, T& v) {
     if (r < w && j < rc) A[int64_t(first + r) * g.k + j0 + j] = v;
   });
