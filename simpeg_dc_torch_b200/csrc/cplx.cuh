@@ -16,7 +16,6 @@ namespace dct {
 // the overloads below must not hide the real ones inside this namespace
 using ::atomicAdd;
 using ::sqrt;
-using ::__shfl_sync;
 
 struct __align__(16) cplx {
   double re, im;
@@ -71,13 +70,6 @@ __host__ __device__ inline cplx sqrt(const cplx& z) {
 __device__ __forceinline__ bool good_pivot(const cplx& v) {
   const double m = fabs(v.re) + fabs(v.im);
   return m > 0.0 && m < INFINITY;
-}
-
-__device__ __forceinline__ cplx inv_sqrt(const cplx& x) { return cplx(1.0) / sqrt(x); }
-
-__device__ __forceinline__ cplx __shfl_sync(unsigned mask, const cplx& v, int src,
-                                            int width = 32) {
-  return cplx(::__shfl_sync(mask, v.re, src, width), ::__shfl_sync(mask, v.im, src, width));
 }
 
 __device__ __forceinline__ void atomicAdd(cplx* p, const cplx& v) {

@@ -260,7 +260,7 @@ k_large_update(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
         return;
       }
     }
-    factor_block<T, kThreads>(F, N, cq, wq, ring, Dv + int64_t(q) * kPanel * kPanel, status, s,
+    factor_block<T, T, kThreads>(F, N, cq, wq, ring, Dv + int64_t(q) * kPanel * kPanel, status, s,
                               b);
   };
   if (tk.t0 < 0) {
@@ -282,30 +282,42 @@ k_large_update(DevSym S, const PanelTask* __restrict__ tasks, T* fronts,
   }
 }
 
-// task: s, p.  D_p^{-1} of the factored diagonal block of panel p of a small
-// general front, written column-major (ld w) at dinv + dinv_off[s] + p*64*64.
+// task: s, p.  The inverse of the factored diagonal block of panel p of a small
+// general front (L, or U^T with its diagonal), written column-major (ld w) at
+// dinv + dinv_off[s] + p*64*64, by the steps of front_small.cuh.
 __global__ void __launch_bounds__(kThreads)
 k_panel_inverse(DevSym S, const PanelTask* __restrict__ tasks, const double* fronts,
                 int64_t front_stride, double* dinv, const int64_t* dinv_off,
                 int64_t dinv_stride) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double* L = reinterpret_cast<double*>(smem_raw);       // ld kDLD
-  double* X = L + kPanel * kDLD;                     // ld kDLD
+  double* L = reinterpret_cast<double*>(smem_raw);
+  constexpr int ld = small_ld<double>(kPanel), kW = kThreads / 32;
+  double* xd = L + ld * kPanel;
   const PanelTask tk = tasks[blockIdx.x];
   const int b = blockIdx.y;
   const int s = tk.s;
   const int N = S.front_n[s];
   const int ns = S.sn_first[s + 1] - S.sn_first[s];
   const int c0 = tk.p * kPanel;
-  const int w = min(kPanel, ns - c0);
-  const double* F = fronts + int64_t(b) * front_stride + S.front_off[s];
-  diag_load<double, kThreads>(F, N, c0, w, L, X);
-  diag_chol_inv<double, kThreads, false>(L, X, nullptr, s, b);
-  double* out = dinv + int64_t(b) * dinv_stride + dinv_off[s] + int64_t(tk.p) * kPanel * kPanel;
-  for (int idx = threadIdx.x; idx < w * w; idx += blockDim.x) {
-    const int r = idx % w, c = idx / w;
-    out[r + c * w] = X[r + c * kDLD];
+  const int w = min(kPanel, ns - c0), nblk = (w + 15) / 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const double* F = fronts + int64_t(b) * front_stride + S.front_off[s] + c0 + int64_t(c0) * N;
+  for (int c = warp; c < w; c += kW)
+    for (int r = c + lane; r < w; r += 32) {
+      const double v = F[r + int64_t(c) * N];
+      L[r + c * ld] = v;
+      if (r == c) xd[c] = 1.0 / v;
+    }
+  __syncthreads();
+  if (warp < nblk) small_leaf_inverse(L, xd, ld, 16 * warp, min(16, w - 16 * warp));
+  for (int i = 1; i < nblk; ++i) {
+    __syncthreads();
+    if (warp < i) small_xblock(L, xd, ld, 16 * i, 16 * warp, w);
   }
+  __syncthreads();
+  double* out = dinv + int64_t(b) * dinv_stride + dinv_off[s] + int64_t(tk.p) * kPanel * kPanel;
+  for (int c = warp; c < w; c += kW)
+    for (int r = lane; r < w; r += 32) out[r + c * w] = xinv(L, xd, ld, r, c);
 }
 
 // ------------------------------------------------------------ supernode inverses
@@ -465,6 +477,36 @@ cudaError_t run_linv(dct_plan* P, cudaStream_t st, const void* fronts, const voi
   return cudaSuccess;
 }
 
+// one launch of single-CTA fronts of order up to n
+template <typename T, typename G>
+struct SmallLaunch {
+  dct_plan* P;
+  const PanelTask* tasks;
+  const void* vals;
+  int vals_dtype;
+  int64_t vals_stride;
+  dim3 grid;
+  cudaStream_t st;
+  static cudaError_t allow(int n) {
+    const cudaError_t e = cudaFuncSetAttribute(
+        k_small_front<T, G, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        static_cast<int>(small_smem<T>(n)));
+    return e != cudaSuccess
+               ? e
+               : cudaFuncSetAttribute(k_small_front<T, G, kThreads / 2>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      static_cast<int>(small_smem<T>(std::min(kSmallNarrow, n))));
+  }
+  cudaError_t operator()(int n) const {
+    const bool narrow = n <= kSmallNarrow;
+    return launch_pdl(narrow ? k_small_front<T, G, kThreads / 2> : k_small_front<T, G, kThreads>,
+                      grid, dim3(narrow ? kThreads / 2 : kThreads), small_smem<T>(n), st, P->ds,
+                      tasks, vals, vals_dtype, vals_stride, static_cast<G*>(P->fronts),
+                      P->front_stride, static_cast<G*>(P->dinv),
+                      static_cast<const int64_t*>(P->d_dinv_off), P->dinv_stride, P->status);
+  }
+};
+
 template <typename T>
 cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
                         int64_t vals_stride, cudaStream_t st) {
@@ -478,17 +520,14 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
   const size_t lu_smem = sizeof(T) * (size_t(small_max) * small_max + small_max);
   const size_t panel_smem = sizeof(T) * (2 * kPanel * kPanelLd);
   // the update kernel's copy ring, or the diagonal block's workspace
-  constexpr int kDiagElems = kDiagSmemElems > kBlockElems<T> ? kDiagSmemElems : kBlockElems<T>;
+  constexpr int kDiagElems = kLuDiagElems > kBlockElems<T> ? kLuDiagElems : kBlockElems<T>;
   constexpr int kUpdateElems = std::max(TilePipe<T, kUT, false>::kElems, kDiagElems);
   const size_t update_smem = sizeof(T) * kUpdateElems;
   // attributes are per device: set them on every call (cheap host calls)
-  e = cudaFuncSetAttribute(k_small_front<T, kThreads>,
-                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(small_smem<T>(small_max)));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_small_front<T, kThreads / 2>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(small_smem<T>(std::min(kSmallNarrow, small_max))));
+  e = SmallLaunch<T, T>::allow(small_max);
+  if constexpr (sizeof(T) == 4) {
+    if (e == cudaSuccess) e = SmallLaunch<double, T>::allow(std::min(small_max, kSmallFrontF64));
+  }
   if constexpr (sizeof(T) == 8) {
     if (e == cudaSuccess && lu)
       e = cudaFuncSetAttribute(k_small_front_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -525,12 +564,13 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
             break;
           }
         }
-        const bool narrow = L.arg <= kSmallNarrow;
-        e = launch_pdl(narrow ? k_small_front<T, kThreads / 2> : k_small_front<T, kThreads>, grid,
-                       dim3(narrow ? kThreads / 2 : kThreads), small_smem<T>(L.arg), st, P->ds, t,
-                       vals, vals_dtype, vals_stride, fronts, P->front_stride,
-                       static_cast<T*>(P->dinv), static_cast<const int64_t*>(P->d_dinv_off),
-                       P->dinv_stride, P->status);
+        SmallLaunch<T, T> go{P, t, vals, vals_dtype, vals_stride, grid, st};
+        if constexpr (sizeof(T) == 4)
+          e = L.arg <= kSmallFrontF64
+                  ? SmallLaunch<double, T>{P, t, vals, vals_dtype, vals_stride, grid, st}(L.arg)
+                  : go(L.arg);
+        else
+          e = go(L.arg);
         if (e != cudaSuccess) return e;
         break;
       }
@@ -588,7 +628,7 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
   if constexpr (sizeof(T) == 8) {
     const int64_t ninv = int64_t(P->inv.tasks.size());
     if (lu && ninv > 0) {
-      const size_t inv_smem = sizeof(T) * kDiagSmemElems;
+      const size_t inv_smem = sizeof(T) * kBlockElems<T>;
       e = cudaFuncSetAttribute(k_panel_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                static_cast<int>(inv_smem));
       if (e == cudaSuccess) e = P->prof.begin(kPanelInverse, 0.0, 0.0, st);

@@ -46,10 +46,13 @@ __device__ __forceinline__ double block_max(double v, double* red) {
   return m;
 }
 
+constexpr int kDLD = kPanel + 1;   // rows and columns free of bank conflicts
+constexpr int kLuDiagElems = 2 * kPanel * kDLD;
+
 // LU of the w x w diagonal block of panel p (columns c0 ..) of a general
 // front (order N): D = [lower from F1 | upper from F2^T], padded to 64 with
 // the identity; writes L (unit) to F1, U^T to F2, L^{-1} to dinv_l and
-// (U^T)^{-1} to dinv_m (w x w, ld w).  Needs kDiagSmemElems doubles at sm.
+// (U^T)^{-1} to dinv_m (w x w, ld w).  Needs kLuDiagElems doubles at sm.
 template <int NT>
 __device__ __noinline__ void lu_diag(double* F1, double* F2, int N, int c0, int w, double* sm,
                                      double* dinv_l, double* dinv_m, int* status, int s, int b,

@@ -472,33 +472,40 @@ constexpr int kBlockElems = small_ld<T>(kPanel) * kPanel + kPanel + 16;
 // N): L is written back (lower part), D^{-1} (w x w, ld w) to inv.  sm:
 // kBlockElems elements.  The blocked steps above took the place of a 64 x 64
 // Cholesky with the inverse formed in three CTA-wide steps per 16 columns.
-template <typename T, int NT>
-__device__ __noinline__ void factor_block(T* Fg, int N, int c0, int w, T* sm, T* inv, int* status,
+// Fronts of G = float are computed in T = double: the block is all latency, and
+// the double tensor cores shorten it (in float, on the FMA units, one took
+// twice as long); only its results are rounded.
+template <typename T, typename G, int NT>
+__device__ __noinline__ void factor_block(G* Fg, int N, int c0, int w, T* sm, G* inv, int* status,
                                           int s, int b) {
   __shared__ int next_tile;
   const int ld = small_ld<T>(kPanel);
   T* xd = sm + ld * kPanel;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int kW = NT / 32;
-  T* D = Fg + c0 + int64_t(c0) * N;
+  G* D = Fg + c0 + int64_t(c0) * N;
   if (tid == 0) next_tile = 0;
   for (int c = warp; c < w; c += kW)
-    for (int r = c + lane; r < w; r += 32) sm[r + c * ld] = D[r + int64_t(c) * N];
+    for (int r = c + lane; r < w; r += 32) sm[r + c * ld] = T(D[r + int64_t(c) * N]);
   __syncthreads();
   small_panel<T, NT>(sm, xd, ld, w, 0, w, &next_tile, status, s, b);
   small_panel_last(sm, xd, ld, 0, w);
   __syncthreads();
   for (int c = warp; c < w; c += kW)
     for (int r = lane; r < w; r += 32) {
-      if (r >= c) D[r + int64_t(c) * N] = sm[r + c * ld];
-      inv[r + c * w] = xinv(sm, xd, ld, r, c);
+      if (r >= c) D[r + int64_t(c) * N] = G(sm[r + c * ld]);
+      inv[r + c * w] = G(xinv(sm, xd, ld, r, c));
     }
 }
 
-template <typename T, int NT>
+// T: what the front is computed in; G: what it is stored in.  Float fronts
+// of up to 160 rows are computed in double, like their diagonal blocks above
+// (and their entries need no rounding before the sums); larger ones in float,
+// which is all that shared memory holds of them.
+template <typename T, typename G, int NT>
 __global__ void __launch_bounds__(NT, (sizeof(T) > 8 ? 256 : 512) / NT)
 k_small_front(DevSym S, const PanelTask* __restrict__ tasks, const void* vals, int vals_dtype,
-              int64_t vals_stride, T* fronts, int64_t front_stride, T* dinv,
+              int64_t vals_stride, G* fronts, int64_t front_stride, G* dinv,
               const int64_t* __restrict__ dinv_off, int64_t dinv_stride, int* status) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ int next_tile;
@@ -512,8 +519,8 @@ k_small_front(DevSym S, const PanelTask* __restrict__ tasks, const void* vals, i
   int32_t* rel_s = reinterpret_cast<int32_t*>(xd + N + 16);   // two maps of N
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr int kW = NT / 32;
-  const T* own = fronts + int64_t(b) * front_stride;
-  T* out = fronts + int64_t(b) * front_stride + S.front_off[s];
+  const G* own = fronts + int64_t(b) * front_stride;
+  G* out = fronts + int64_t(b) * front_stride + S.front_off[s];
 
   // Assembly.  Its cost is the latency of dependent loads, so what does not
   // depend on the predecessor (the zeros, the row maps, the children's
@@ -530,7 +537,7 @@ k_small_front(DevSym S, const PanelTask* __restrict__ tasks, const void* vals, i
   }
   const int ch0 = S.child_ptr[s], ch1 = S.child_ptr[s + 1];
   int nbc[2] = {0, 0}, ncc[2] = {0, 0};
-  const T* upd[2] = {nullptr, nullptr};
+  const G* upd[2] = {nullptr, nullptr};
   auto meet = [&](int ci, int u) {   // child ci: its size, place and row map
     const int c = S.child[ci];
     const int nsc = S.sn_first[c + 1] - S.sn_first[c];
@@ -575,12 +582,12 @@ k_small_front(DevSym S, const PanelTask* __restrict__ tasks, const void* vals, i
         for (int q = 0; q < kAddCols; ++q) to[q] = j0 + q * kW < nb ? rel[j0 + q * kW] * ld : 0;
 #pragma unroll 1
         for (int i = j0 + lane; i < nb + lane; i += 32) {
-          const T* src = upd[u] + min(i, nb - 1) + int64_t(j0) * nc;
+          const G* src = upd[u] + min(i, nb - 1) + int64_t(j0) * nc;
           const int ri = i < nb ? rel[i] : 0;
           T v[kAddCols];
 #pragma unroll
           for (int q = 0; q < kAddCols; ++q)
-            v[q] = i < nb && j0 + q * kW <= i ? src[q * kW * nc] : T(0);
+            v[q] = i < nb && j0 + q * kW <= i ? T(src[q * kW * nc]) : T(0);
 #pragma unroll
           for (int q = 0; q < kAddCols; ++q)
             if (i < nb && j0 + q * kW <= i) F[ri + to[q]] += v[q];
@@ -609,12 +616,12 @@ k_small_front(DevSym S, const PanelTask* __restrict__ tasks, const void* vals, i
   // inverses, whole w x w blocks
   for (int c = warp; c < N; c += kW)
 #pragma unroll 4
-    for (int r = c + lane; r < N; r += 32) out[r + c * N] = F[r + c * ld];
-  T* inv = dinv + int64_t(b) * dinv_stride + dinv_off[s];
+    for (int r = c + lane; r < N; r += 32) out[r + c * N] = G(F[r + c * ld]);
+  G* inv = dinv + int64_t(b) * dinv_stride + dinv_off[s];
   for (int c = warp; c < ns; c += kW) {
     const int c0 = c / kPanel * kPanel, w = min(kPanel, ns - c0);
-    T* dst = inv + int64_t(c0) * kPanel + int64_t(c - c0) * w;
-    for (int r = lane; r < w; r += 32) dst[r] = xinv(F, xd, ld, c0 + r, c);
+    G* dst = inv + int64_t(c0) * kPanel + int64_t(c - c0) * w;
+    for (int r = lane; r < w; r += 32) dst[r] = G(xinv(F, xd, ld, c0 + r, c));
   }
 }
 

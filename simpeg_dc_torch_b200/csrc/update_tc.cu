@@ -48,7 +48,7 @@
 #include <algorithm>
 
 #include "dct_internal.h"
-#include "factor_diag.cuh"
+#include "front_small.cuh"
 #include "tc_common.cuh"
 
 namespace dct {
@@ -69,8 +69,8 @@ constexpr int kUTileBytes = kTcM * kTcN * 4;   // the output tile, staged
 constexpr int kUBarBytes = 256;             // mbarriers, TMEM address, abort word
 constexpr size_t kUSmem = size_t(kUStages) * kUStageBytes + kUTileBytes + kUBarBytes;
 static_assert(kUAcc * 128 <= 512, "TMEM columns of one SM");
-static_assert(size_t(kUStages) * kUStageBytes >= sizeof(float) * kDiagSmemElems,
-              "the ring also holds factor_diag's workspace");
+static_assert(size_t(kUStages) * kUStageBytes >= sizeof(double) * kBlockElems<double>,
+              "the ring also holds factor_block's workspace");
 static_assert(kUSmem <= 227 * 1024, "shared memory of one CTA");
 static_assert((2 * kUStages + 2 * kUAcc + 1) * 8 + 8 <= kUBarBytes,
               "barriers, the TMEM slot and the abort word");
@@ -382,8 +382,8 @@ k_update_tc(DevSym S, const PanelTask* __restrict__ tasks, float* fronts,
   float* Dv = dinv + int64_t(b) * dinv_stride + dinv_off[s];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tk.t0 < 0) {
-    factor_diag<float, kUThreads>(F, N, c0, w, reinterpret_cast<float*>(smem_raw),
-                                  Dv + int64_t(tk.p) * kPanel * kPanel, status, s, b);
+    factor_block<double, float, kUThreads>(F, N, c0, w, reinterpret_cast<double*>(smem_raw),
+                                   Dv + int64_t(tk.p) * kPanel * kPanel, status, s, b);
     return;
   }
   const UpdateRange R = update_range(tk.p, ns, N, bpan);
@@ -527,9 +527,9 @@ k_update_tc(DevSym S, const PanelTask* __restrict__ tasks, float* fronts,
   if (warp == 1) tmem_dealloc(tmem, kUAcc * 128);
   if (all_ok && tk.t0 == 0 && tk.t1 == 0 && base < ns) {
     __syncthreads();   // this CTA's updates of the block are complete
-    factor_diag<float, kUThreads>(F, N, base, min(kPanel, ns - base),
-                                  reinterpret_cast<float*>(smem_raw),
-                                  Dv + int64_t(tk.p + 1) * kPanel * kPanel, status, s, b);
+    factor_block<double, float, kUThreads>(F, N, base, min(kPanel, ns - base),
+                                   reinterpret_cast<double*>(smem_raw),
+                                   Dv + int64_t(tk.p + 1) * kPanel * kPanel, status, s, b);
   }
 }
 
