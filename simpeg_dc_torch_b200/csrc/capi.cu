@@ -868,9 +868,23 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
       (rc = upload(P, S.amap_e, &D.amap_e)) || (rc = upload(P, S.amap_pos, &D.amap_pos)) ||
       (rc = upload(P, S.child_ptr, &D.child_ptr)) || (rc = upload(P, S.child, &D.child)) ||
       (rc = upload(P, S.rel_ptr, &D.rel_ptr)) || (rc = upload(P, S.rel, &D.rel)) ||
-      (rc = upload(P, S.perm, &D.perm)) || (rc = upload(P, S.iperm, &D.iperm)) ||
-      (rc = upload(P, S.in_crow, &D.crow)) || (rc = upload(P, S.in_col, &D.col)))
+      (rc = upload(P, S.perm, &D.perm)) || (rc = upload(P, S.iperm, &D.iperm)))
     return bail(rc);
+  if (dtype == DCT_F32) {
+    std::vector<int32_t> pptr(S.n + 1, 0), pcol, pent;
+    pcol.reserve(S.in_col.size());
+    pent.reserve(S.in_col.size());
+    for (int i = 0; i < S.n; ++i) {
+      for (int64_t e = S.in_crow[S.perm[i]]; e < S.in_crow[S.perm[i] + 1]; ++e) {
+        pcol.push_back(S.iperm[S.in_col[e]]);
+        pent.push_back(static_cast<int32_t>(e));
+      }
+      pptr[i + 1] = static_cast<int32_t>(pent.size());
+    }
+    if ((rc = upload(P, pptr, &D.pptr)) || (rc = upload(P, pcol, &D.pcol)) ||
+        (rc = upload(P, pent, &D.pent)))
+      return bail(rc);
+  }
   P->tune = resolve_tuning(dtype, tuning);
   const int small_max = P->tune.small_front_max;
   P->update_bpan = plan_update_block(dtype, P->tune);
@@ -926,6 +940,18 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
   }
   account_factor(S, &P->fact, double(esize(dtype)), update_tile(dtype),
                  P->update_bpan, dtype == DCT_F32);
+  if (dtype == DCT_F32) {
+    // the supernodes without a single-panel task
+    std::vector<char> small(S.nsuper, 0);
+    for (const Launch& l : P->fwd.launches)
+      if (l.kind == dct::kFwdSmall)
+        for (int64_t q = l.first; q < l.first + l.count; ++q) small[P->fwd.tasks[q].s] = 1;
+    std::vector<int32_t> tc;
+    for (int s = 0; s < S.nsuper; ++s)
+      if (!small[s]) tc.push_back(s);
+    if ((rc = upload(P, tc, &P->d_tc))) return bail(rc);
+    P->n_tc = static_cast<int32_t>(tc.size());
+  }
   account_solve(S, &P->fwd, double(esize(dtype)));
   account_solve(S, &P->bwd, double(esize(dtype)));
   if ((rc = upload_schedule(P, &P->fact)) || (rc = upload_schedule(P, &P->fwd)) ||
@@ -934,7 +960,7 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
     return bail(rc);
   const size_t es = esize(dtype);
   P->front_stride = S.front_total;
-  const size_t work = size_t(nbatch) * S.n * max_rhs;
+  const size_t work = size_t(nbatch) * S.n * (dtype == DCT_F32 ? dct::rhs_ld(max_rhs) : max_rhs);
   void* p = nullptr;
   if ((rc = alloc(P, es * S.front_total * nbatch, &P->fronts, "front storage")))
     return bail(rc);
@@ -947,9 +973,10 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
   if ((rc = alloc(P, es * work, &P->bufA, "work buffer A"))) return bail(rc);
   if ((rc = alloc(P, es * work, &P->bufB, "work buffer B"))) return bail(rc);
   if (dtype == DCT_F32) {
-    if ((rc = alloc(P, 8 * work, &p, "refinement iterate"))) return bail(rc);
+    const size_t work64 = 8 * size_t(nbatch) * S.n * max_rhs;
+    if ((rc = alloc(P, work64, &p, "refinement iterate"))) return bail(rc);
     P->x64 = static_cast<double*>(p);
-    if ((rc = alloc(P, 8 * work, &p, "refinement rhs"))) return bail(rc);
+    if ((rc = alloc(P, work64, &p, "refinement rhs"))) return bail(rc);
     P->b64 = static_cast<double*>(p);
     if ((rc = alloc(P, 8 * size_t(nbatch) * S.nnz_in, &p, "float64 values")))
       return bail(rc);
@@ -1100,13 +1127,9 @@ namespace {
 // f32 plans: solve bp -> xp (both float64, permuted) with refinement.
 int solve_refined(dct_plan* P, const double* bp, int64_t bstride, int k,
                   double* xp, cudaStream_t st) {
-  const int n = P->sym.n;
-  const int64_t per = int64_t(n) * k;
   DCT_CUDA(cudaMemsetAsync(P->resid_bits, 0, 16, st), "memset");
   DCT_CUDA(cudaMemsetAsync(P->ir, 0, sizeof(dct::IrState), st), "memset");
-  DCT_CUDA(dct::launch_convert_any(bp, DCT_F64, bstride, per, P->nbatch, P->bufA,
-                                   DCT_F32, st),
-           "rhs conversion");
+  DCT_CUDA(dct::launch_rhs_to_float(P, bp, bstride, k, st), "rhs conversion");
   DCT_CUDA(dct::run_solve_f32(P, k, st), "solve launch");
   DCT_CUDA(dct::launch_ir_update(P, xp, k, 1, st), "refinement update");
   // corrections until the estimated error is below the tolerance, the

@@ -45,8 +45,12 @@ struct DevSym {
   const int32_t* rel;
   const int32_t* perm;
   const int32_t* iperm;
-  const int32_t* crow;   // input pattern (refinement residuals)
-  const int32_t* col;
+  // float32 plans (refinement residuals): the input pattern in the permuted
+  // order -- row pointers, permuted columns, and each entry's place among the
+  // values
+  const int32_t* pptr;
+  const int32_t* pcol;
+  const int32_t* pent;
 };
 
 // One launch of a factor or solve schedule: `count` tasks from `first`.
@@ -262,6 +266,8 @@ struct dct_plan {
   unsigned long long* resid_bits = nullptr;  // device: max|r|, max|b|
   int factored = 0;
   int64_t stamp = 0;
+  const int32_t* d_tc = nullptr;   // f32 plans: supernodes solved by the tensor-core
+  int32_t n_tc = 0;                //   products, and how many they are
   dct::ImgArgs img{};              // f32 plans: split panel images (large fronts)
   dct_tuning tune{};               // schedule shapes (resolved, no zero fields)
   int ir_iters = 2;                // most refinement iterations of f32 plans
@@ -339,6 +345,11 @@ cudaError_t launch_perm_out_any(const void* src, int src_dtype,
 cudaError_t launch_convert_any(const void* src, int src_dtype, int64_t sstride,
                                int64_t count, int nbatch, void* dst,
                                int dst_dtype, cudaStream_t st);
+// floats in a row of the float32 plans' right-hand sides (see solve.cu)
+inline int rhs_ld(int k) { return (k + 3) & ~3; }
+// b (float64, permuted) -> buffer A of a float32 plan
+cudaError_t launch_rhs_to_float(dct_plan* P, const double* b, int64_t bstride, int k,
+                                cudaStream_t st);
 cudaError_t launch_residual(dct_plan* P, const double* b, int64_t bstride,
                             const double* x, int k, cudaStream_t st);
 cudaError_t launch_ir_update(dct_plan* P, double* x, int k, int first,

@@ -507,9 +507,9 @@ __global__ void __launch_bounds__(NT, (sizeof(T) > 8 ? 256 : 512) / NT)
 k_small_front(DevSym S, const PanelTask* __restrict__ tasks, const void* vals, int vals_dtype,
               int64_t vals_stride, G* fronts, int64_t front_stride, G* dinv,
               const int64_t* __restrict__ dinv_off, int64_t dinv_stride, int* status) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(16) unsigned char front_raw[];
   __shared__ int next_tile;
-  T* F = reinterpret_cast<T*>(smem_raw);
+  T* F = reinterpret_cast<T*>(front_raw);
   const int s = tasks[blockIdx.x].s;
   const int b = blockIdx.y;
   const int N = S.front_n[s];

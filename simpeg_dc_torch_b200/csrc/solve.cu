@@ -207,44 +207,90 @@ __global__ void k_convert(const TI* __restrict__ src, int64_t sstride, int64_t c
 }
 
 // ------------------------------------------------------------ refinement
-// right-hand sides per thread of the refinement residual (1, 2, 4 or 8)
-#ifndef DCT_RESIDUAL_RHS
-#define DCT_RESIDUAL_RHS 4
-#endif
-constexpr int kResidualRhs = DCT_RESIDUAL_RHS;
+// The float32 work buffers hold their right-hand sides in rows of rhs_ld(k)
+// floats, k rounded up to four, the columns beyond k zero: whatever k is, the
+// substitution copies and reduces 16 bytes at a time.  The kernels between
+// those rows and the callers' float64 rows of k take four columns per thread;
+// V = 2 where the float64 rows are 16-byte aligned, else 1.
 
-// r = b - A x in float64 (permuted order), stored as float into the f32 work
-// buffer, with max|r| and max|b| folded into maxbits[0..1] (the refinement
-// state's rmax, bmax).  Threads walk the rows in the permuted order: the
-// nested dissection keeps each subdomain's rows together, and b and r move
-// as contiguous rows (walking the matrix's own order measured 11 % slower
-// on the 269,001-node benchmark).
+// up to four doubles of a row whose columns from j on number `left`
+template <int V>
+__device__ __forceinline__ void load_quad(const double* p, int left, double (&v)[4]) {
+#pragma unroll
+  for (int h = 0; h < 4; h += V) {
+    if constexpr (V == 2) {
+      const double2 q = h < left ? *reinterpret_cast<const double2*>(p + h) : make_double2(0, 0);
+      v[h] = q.x;
+      v[h + 1] = q.y;
+    } else {
+      v[h] = h < left ? p[h] : 0.0;
+    }
+  }
+}
 
-__global__ void k_residual(DevSym S, const double* __restrict__ vals,
-                           int64_t vals_stride, const double* __restrict__ b,
-                           int64_t bstride, const double* __restrict__ x, int n,
-                           int k, float* __restrict__ r32,
-                           unsigned long long* __restrict__ maxbits, const int* skip) {
+// b (float64, n x k) -> the float32 right-hand sides
+template <int V>
+__global__ void k_rhs_to_float(const double* __restrict__ b, int64_t bstride, int n, int k, int kp,
+                               float* __restrict__ r32) {
+  const int kq = kp / 4;
+  const int64_t total = int64_t(n) * kq;
+  const double* Bv = b + int64_t(blockIdx.y) * bstride;
+  float4* R = reinterpret_cast<float4*>(r32) + int64_t(blockIdx.y) * total;
+  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
+       idx += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t i = idx / kq;
+    const int j = static_cast<int>(idx - i * kq) * 4;
+    double v[4];
+    load_quad<V>(Bv + i * k + j, k - j, v);
+    R[idx] = make_float4(float(v[0]), float(v[1]), float(v[2]), float(v[3]));
+  }
+}
+
+// r = b - A x in float64 (permuted order), stored as float, with max|r| and
+// max|b| folded into maxbits[0..1] (the refinement state's rmax, bmax).
+// Threads walk the rows in the permuted order: the nested dissection keeps
+// each subdomain's rows together, and b and r move as contiguous rows (walking
+// the matrix's own order measured 11 % slower on the 269,001-node benchmark).
+// The pattern is kept in that order (pptr, pcol, and pent, the place of each
+// entry's value), so that an x is two dependent loads away and not four.
+// Measured, 56,525 nodes x 12 systems x 186 right-hand sides: 0.71 ms; one column
+// per thread through perm, crow, col and iperm took 1.38 ms.
+template <int V>
+__global__ void k_residual(DevSym S, const double* __restrict__ vals, int64_t vals_stride,
+                           const double* __restrict__ b, int64_t bstride,
+                           const double* __restrict__ x, int n, int k, int kp,
+                           float* __restrict__ r32, unsigned long long* __restrict__ maxbits,
+                           const int* skip) {
   if (ir_skip(skip)) return;
   const int bb = blockIdx.y;
-  const double* V = vals + int64_t(bb) * vals_stride;
+  const double* W = vals + int64_t(bb) * vals_stride;
   const double* X = x + int64_t(bb) * n * k;
   const double* Bv = b + int64_t(bb) * bstride;
-  float* R = r32 + int64_t(bb) * n * k;
-  double rmax = 0.0, bmax = 0.0;
   // n * k < 2^31 (checked at launch): 32-bit index arithmetic
-  const int total = n * k;
+  const int kq = kp / 4, total = n * kq;
+  float4* R = reinterpret_cast<float4*>(r32) + int64_t(bb) * total;
+  double rmax = 0.0, bmax = 0.0;
   for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += gridDim.x * blockDim.x) {
-    const int i = idx / k;
-    const int j = idx - i * k;
-    const int orow = S.perm[i];
-    double acc = Bv[idx];
-    bmax = fmax(bmax, fabs(acc));
-    for (int e = S.crow[orow]; e < S.crow[orow + 1]; ++e)
-      acc -= V[e] * X[int64_t(S.iperm[S.col[e]]) * k + j];
-    R[idx] = static_cast<float>(acc);
-    rmax = fmax(rmax, fabs(acc));
+    const int i = idx / kq, j = (idx - i * kq) * 4, left = k - j;
+    double acc[4];
+    load_quad<V>(Bv + int64_t(i) * k + j, left, acc);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) bmax = fmax(bmax, fabs(acc[h]));
+    const int e1 = S.pptr[i + 1];
+#pragma unroll 4
+    for (int e = S.pptr[i]; e < e1; ++e) {
+      const double a = W[S.pent[e]];
+      double v[4];
+      load_quad<V>(X + int64_t(S.pcol[e]) * k + j, left, v);
+#pragma unroll
+      for (int h = 0; h < 4; ++h) acc[h] -= a * v[h];
+    }
+    R[idx] = make_float4(float(acc[0]), left > 1 ? float(acc[1]) : 0.f,
+                         left > 2 ? float(acc[2]) : 0.f, left > 3 ? float(acc[3]) : 0.f);
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (h < left) rmax = fmax(rmax, fabs(acc[h]));
   }
   // non-negative doubles order like their bit patterns
   for (int o = 16; o > 0; o >>= 1) {
@@ -257,85 +303,40 @@ __global__ void k_residual(DevSym S, const double* __restrict__ vals,
   }
 }
 
-// The same with RJ = 2, 4 or 8 consecutive right-hand sides per thread (k a
-// multiple of RJ, rows 16-byte aligned): the row's pattern, permutation and
-// values are read once for RJ outputs, and x, b and r move as 16-byte vectors.
-template <int RJ>
-__global__ void k_residual_vec(DevSym S, const double* __restrict__ vals,
-                               int64_t vals_stride, const double* __restrict__ b,
-                               int64_t bstride, const double* __restrict__ x, int n,
-                               int k, float* __restrict__ r32,
-                               unsigned long long* __restrict__ maxbits, const int* skip) {
-  static_assert(RJ == 2 || RJ == 4 || RJ == 8, "2, 4 or 8 right-hand sides per thread");
-  if (ir_skip(skip)) return;
-  const int bb = blockIdx.y;
-  const double* V = vals + int64_t(bb) * vals_stride;
-  const double* X = x + int64_t(bb) * n * k;
-  const double* Bv = b + int64_t(bb) * bstride;
-  float* R = r32 + int64_t(bb) * n * k;
-  double rmax = 0.0, bmax = 0.0;
-  const int kq = k / RJ;
-  // n * k < 2^31 (checked at launch): 32-bit index arithmetic
-  const int total = n * kq;
-  for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-       idx += gridDim.x * blockDim.x) {
-    const int i = idx / kq;
-    const int o = i * k + (idx - i * kq) * RJ;   // element (i, j)
-    const int orow = S.perm[i];
-    double acc[RJ];
-#pragma unroll
-    for (int h = 0; h < RJ; h += 2) {
-      const double2 v = *reinterpret_cast<const double2*>(Bv + o + h);
-      acc[h] = v.x;
-      acc[h + 1] = v.y;
-    }
-#pragma unroll
-    for (int h = 0; h < RJ; ++h) bmax = fmax(bmax, fabs(acc[h]));
-    const int j = o - i * k;
-    for (int e = S.crow[orow]; e < S.crow[orow + 1]; ++e) {
-      const double a = V[e];
-      const double* xr = X + S.iperm[S.col[e]] * k + j;
-#pragma unroll
-      for (int h = 0; h < RJ; h += 2) {
-        const double2 v = *reinterpret_cast<const double2*>(xr + h);
-        acc[h] -= a * v.x;
-        acc[h + 1] -= a * v.y;
-      }
-    }
-    if constexpr (RJ == 2) {
-      *reinterpret_cast<float2*>(R + o) = make_float2(float(acc[0]), float(acc[1]));
-    } else {
-#pragma unroll
-      for (int h = 0; h < RJ; h += 4)
-        *reinterpret_cast<float4*>(R + o + h) = make_float4(
-            float(acc[h]), float(acc[h + 1]), float(acc[h + 2]), float(acc[h + 3]));
-    }
-#pragma unroll
-    for (int h = 0; h < RJ; ++h) rmax = fmax(rmax, fabs(acc[h]));
-  }
-  for (int off = 16; off > 0; off >>= 1) {
-    rmax = fmax(rmax, __shfl_xor_sync(0xffffffffu, rmax, off));
-    bmax = fmax(bmax, __shfl_xor_sync(0xffffffffu, bmax, off));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(&maxbits[0], __double_as_longlong(rmax));
-    atomicMax(&maxbits[1], __double_as_longlong(bmax));
-  }
-}
-
 // x = c (first) or x += c, folding max|c| and max|x| into the refinement
-// state (corrections only)
-__global__ void k_ir_update(const float* __restrict__ c, int64_t count,
+// state (corrections only); rows: nbatch n of them
+template <int V>
+__global__ void k_ir_update(const float* __restrict__ c, int64_t rows, int k, int kp,
                             double* __restrict__ x, int first, IrState* ir) {
   if (!first && ir_skip(&ir->done)) return;
+  const int kq = kp / 4;
+  const int64_t total = rows * kq;
   double cmax = 0.0, xmax = 0.0;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < count;
-       i += int64_t(gridDim.x) * blockDim.x) {
-    const double ci = double(c[i]);
-    const double xi = first ? ci : x[i] + ci;
-    x[i] = xi;
-    cmax = fmax(cmax, fabs(ci));
-    xmax = fmax(xmax, fabs(xi));
+  for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
+       idx += int64_t(gridDim.x) * blockDim.x) {
+    const int64_t i = idx / kq;
+    const int j = static_cast<int>(idx - i * kq) * 4, left = k - j;
+    const float4 f = reinterpret_cast<const float4*>(c)[idx];
+    const double ci[4] = {f.x, f.y, f.z, f.w};
+    double* xr = x + i * k + j;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    if (!first) load_quad<V>(xr, left, v);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      v[h] = first ? ci[h] : v[h] + ci[h];
+      if (h < left) {
+        cmax = fmax(cmax, fabs(ci[h]));
+        xmax = fmax(xmax, fabs(v[h]));
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 4; h += V)
+      if (h < left) {
+        if constexpr (V == 2)
+          *reinterpret_cast<double2*>(xr + h) = make_double2(v[h], v[h + 1]);
+        else
+          xr[h] = v[h];
+      }
   }
   if (first) return;
   for (int o = 16; o > 0; o >>= 1) {
@@ -347,6 +348,17 @@ __global__ void k_ir_update(const float* __restrict__ c, int64_t count,
     atomicMax(&ir->cmax, __double_as_longlong(cmax));
     atomicMax(&ir->xmax, __double_as_longlong(xmax));
   }
+}
+
+// zeros in the rows of the supernodes `sn` (one CTA each per system): those
+// whose products accumulate
+__global__ void k_clear_rows(DevSym S, const int32_t* __restrict__ sn, float* __restrict__ buf,
+                             int64_t stride, int k) {
+  const int s = sn[blockIdx.x];
+  float4* p = reinterpret_cast<float4*>(buf + int64_t(blockIdx.y) * stride +
+                                        int64_t(S.sn_first[s]) * k);
+  const int64_t count = int64_t(S.sn_first[s + 1] - S.sn_first[s]) * k / 4;
+  for (int64_t i = threadIdx.x; i < count; i += blockDim.x) p[i] = make_float4(0, 0, 0, 0);
 }
 
 // One thread, after correction `iter` (1-based): the estimate of the error
@@ -479,9 +491,15 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
     g.fronts = fac[pass];
     g.dinv = dv[pass];
     g.linv = lv[pass];
-    if (kTc) {
-      e = cudaMemsetAsync(sc == &P->fwd ? static_cast<void*>(bufB) : static_cast<void*>(bufA),
-                          0, work, st);
+    if constexpr (kTc) {
+      // the rows that the tensor-core products accumulate into
+      T* buf = sc == &P->fwd ? bufB : bufA;
+      if (P->n_tc == P->sym.nsuper)
+        e = cudaMemsetAsync(buf, 0, work, st);
+      else if (P->n_tc > 0)
+        k_clear_rows<<<dim3(static_cast<unsigned>(P->n_tc), P->nbatch), kThreads, 0, st>>>(
+            P->ds, P->d_tc, buf, int64_t(P->sym.n) * k, k);
+      if (e == cudaSuccess) e = cudaGetLastError();
       if (e != cudaSuccess) return e;
     }
     for (size_t li = 0; li < sc->launches.size(); ++li) {
@@ -531,10 +549,11 @@ cudaError_t run_solve_c128(dct_plan* P, cplx* xa, int k, cudaStream_t st) {
   return solve_impl<cplx>(P, xa, static_cast<cplx*>(P->bufB), k, st);
 }
 
-// f32 plans: right-hand side in P->bufA (float, A), P->bufB (B).
+// f32 plans: right-hand side in P->bufA (float, A), P->bufB (B), rows of
+// rhs_ld(k).
 cudaError_t run_solve_f32(dct_plan* P, int k, cudaStream_t st) {
-  return solve_impl<float>(P, static_cast<float*>(P->bufA),
-                           static_cast<float*>(P->bufB), k, st);
+  return solve_impl<float>(P, static_cast<float*>(P->bufA), static_cast<float*>(P->bufB),
+                           rhs_ld(k), st);
 }
 
 cudaError_t launch_perm_in_any(const void* b, int b_dtype, int64_t bstride,
@@ -606,42 +625,40 @@ cudaError_t launch_convert_any(const void* src, int src_dtype, int64_t sstride,
   return cudaGetLastError();
 }
 
+// rows of k doubles can be read two at a time
+static bool even_rows(const double* p, int64_t stride, int k) {
+  return k % 2 == 0 && stride % 2 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+}
+
+cudaError_t launch_rhs_to_float(dct_plan* P, const double* b, int64_t bstride, int k,
+                                cudaStream_t st) {
+  const int n = P->sym.n, kp = rhs_ld(k);
+  auto fn = even_rows(b, bstride, k) ? k_rhs_to_float<2> : k_rhs_to_float<1>;
+  fn<<<grid1d(int64_t(n) * kp / 4, P->nbatch), kThreads, 0, st>>>(b, bstride, n, k, kp,
+                                                                 static_cast<float*>(P->bufA));
+  return cudaGetLastError();
+}
+
 cudaError_t launch_residual(dct_plan* P, const double* b, int64_t bstride,
                             const double* x, int k, cudaStream_t st) {
-  const int n = P->sym.n;
+  const int n = P->sym.n, kp = rhs_ld(k);
   if (int64_t(n) * k >= (int64_t(1) << 31)) return cudaErrorInvalidValue;
   const int64_t nnz = static_cast<int64_t>(P->sym.nnz_in);
-  float* r = static_cast<float*>(P->bufA);
-  // vector rows: k and the batch stride a multiple of kResidualRhs, 16-byte
-  // aligned b and x (buffer A comes from cudaMalloc)
-  const bool vec = kResidualRhs > 1 && k % kResidualRhs == 0 && bstride % kResidualRhs == 0 &&
-                   (reinterpret_cast<uintptr_t>(b) & 15) == 0 &&
-                   (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  if (vec) {
-    dim3 g = grid1d(int64_t(n) * (k / kResidualRhs), P->nbatch);
-    if (kResidualRhs == 2)
-      k_residual_vec<2><<<g, kThreads, 0, st>>>(P->ds, P->vals64, nnz, b, bstride, x, n, k, r,
-                                                &P->ir->rmax, &P->ir->done);
-    else if (kResidualRhs == 4)
-      k_residual_vec<4><<<g, kThreads, 0, st>>>(P->ds, P->vals64, nnz, b, bstride, x, n, k, r,
-                                                &P->ir->rmax, &P->ir->done);
-    else
-      k_residual_vec<8><<<g, kThreads, 0, st>>>(P->ds, P->vals64, nnz, b, bstride, x, n, k, r,
-                                                &P->ir->rmax, &P->ir->done);
-  } else {
-    dim3 g = grid1d(int64_t(n) * k, P->nbatch);
-    k_residual<<<g, kThreads, 0, st>>>(P->ds, P->vals64, nnz, b, bstride, x, n, k, r,
-                                       &P->ir->rmax, &P->ir->done);
-  }
+  auto fn = even_rows(b, bstride, k) && even_rows(x, int64_t(n) * k, k) ? k_residual<2>
+                                                                        : k_residual<1>;
+  fn<<<grid1d(int64_t(n) * kp / 4, P->nbatch), kThreads, 0, st>>>(
+      P->ds, P->vals64, nnz, b, bstride, x, n, k, kp, static_cast<float*>(P->bufA), &P->ir->rmax,
+      &P->ir->done);
   return cudaGetLastError();
 }
 
 cudaError_t launch_ir_update(dct_plan* P, double* x, int k, int first,
                              cudaStream_t st) {
-  const int64_t count = int64_t(P->nbatch) * P->sym.n * k;
-  dim3 g = grid1d(count, 1);
-  k_ir_update<<<g, kThreads, 0, st>>>(static_cast<const float*>(P->bufA), count,
-                                      x, first, P->ir);
+  const int kp = rhs_ld(k);
+  const int64_t rows = int64_t(P->nbatch) * P->sym.n;
+  auto fn = even_rows(x, 0, k) ? k_ir_update<2> : k_ir_update<1>;
+  fn<<<grid1d(rows * (kp / 4), 1), kThreads, 0, st>>>(static_cast<const float*>(P->bufA), rows, k,
+                                                      kp, x, first, P->ir);
   return cudaGetLastError();
 }
 

@@ -11,10 +11,9 @@
 //
 // A task covers one 128-row tile of the output and a K range [k0, k1); every
 // task adds its product into the destination rows -- one bulk f32 reduction
-// per row (cp.reduce.async.bulk) when the rows are 16-byte aligned, float
-// atomics otherwise -- so K ranges can be split over tasks, and the
-// destination rows of the two inverse products are cleared before the pass
-// that writes them (see solve.cu).  tcgen05.mma kind::tf32
+// per row (cp.reduce.async.bulk; k is a multiple of 4, see solve.cu) -- so K
+// ranges can be split over tasks, and the destination rows of the two inverse
+// products are cleared before the pass that writes them.  tcgen05.mma kind::tf32
 // with the 3xTF32 split (hi*hi + hi*lo + lo*hi: Markidis et al. 2018; Ootomo
 // and Yokota 2022) accumulates in TMEM.  Operands move in K stages of 16:
 // cp.async copies the float32 values of stage i+2 into a two-deep raw ring
@@ -73,11 +72,6 @@ constexpr int kRawBBytes = kStK * kRawBld * 4;
 constexpr int kRawBytes = kRawABytes + kRawBBytes;
 constexpr size_t kSolveTcSmem = kSets * size_t(kSplitBytes) + kRaw * size_t(kRawBytes) + 64;
 constexpr int kCtasPerSm = DCT_TC_CTAS_PER_SM;
-// output rows leave by bulk reductions (1) or float atomics (0)
-#ifndef DCT_TC_BULK_REDUCE
-#define DCT_TC_BULK_REDUCE 1
-#endif
-constexpr bool kTcBulkReduce = DCT_TC_BULK_REDUCE != 0;
 static_assert(kCtasPerSm * (kSolveTcSmem + 1024) <= 233472, "CTAs per SM");
 static_assert(kRawABytes >= kTcM * kStK * 4, "raw A holds both layouts");
 static_assert(64 * (kStN + 4) * 4 <= kSets * kSplitBytes + kRaw * kRawBytes,
@@ -159,7 +153,6 @@ __global__ void __launch_bounds__(kNT, kCtasPerSm) k_solve_tc(SolveArgs<float> g
   bool ok = true;
   constexpr int kPerA = kTcM * kStK / kNT;          // 8 values
   constexpr int kPerB = kStN * kStK / 4 / kNT;      // 4 float4
-  const bool vec4 = (g.k & 3) == 0;   // 16-byte aligned rows
   // stage st's float32 values -> raw slot st % kRaw (one commit group)
   auto issue_stage = [&](int st) {
     unsigned char* raw = smem_raw + kSets * kSplitBytes + (st % kRaw) * kRawBytes;
@@ -188,37 +181,20 @@ __global__ void __launch_bounds__(kNT, kCtasPerSm) k_solve_tc(SolveArgs<float> g
                                  : (roff + m) + int64_t(kg) * ld;
       cp_async4(rA + d, valid ? M + idx : M, valid ? 4 : 0);
     }
-    if (vec4) {
-      // whole 16-byte quads: kc is a multiple of 4 when k is
+    // whole 16-byte quads: k is a multiple of 4
 #pragma unroll
-      for (int u = 0; u < kStK * kStN / 4 / kNT; ++u) {
-        const int q = tid + u * kNT;
-        const int kl = q / (kStN / 4), n = (q % (kStN / 4)) * 4;
-        const bool valid = kl < kw && n < kc;
-        const float* src = X;
-        if (valid) {
-          const int kg = kb + kl;
-          const int64_t row = MODE == kModeBwdGemm ? int64_t(__ldg(rows + ns + kg))
-                                                   : int64_t(first + kg);
-          src = X + row * g.k + j0 + n;
-        }
-        cp_async16(rB + kl * kRawBld + n, src, valid ? 16 : 0);
+    for (int u = 0; u < kStK * kStN / 4 / kNT; ++u) {
+      const int q = tid + u * kNT;
+      const int kl = q / (kStN / 4), n = (q % (kStN / 4)) * 4;
+      const bool valid = kl < kw && n < kc;
+      const float* src = X;
+      if (valid) {
+        const int kg = kb + kl;
+        const int64_t row = MODE == kModeBwdGemm ? int64_t(__ldg(rows + ns + kg))
+                                                 : int64_t(first + kg);
+        src = X + row * g.k + j0 + n;
       }
-    } else {
-#pragma unroll 4
-      for (int u = 0; u < kStK * kStN / kNT; ++u) {
-        const int q = tid + u * kNT;
-        const int kl = q / kStN, n = q % kStN;
-        const bool valid = kl < kw && n < kc;
-        const float* src = X;
-        if (valid) {
-          const int kg = kb + kl;
-          const int64_t row = MODE == kModeBwdGemm ? int64_t(__ldg(rows + ns + kg))
-                                                   : int64_t(first + kg);
-          src = X + row * g.k + j0 + n;
-        }
-        cp_async4(rB + kl * kRawBld + n, src, valid ? 4 : 0);
-      }
+      cp_async16(rB + kl * kRawBld + n, src, valid ? 16 : 0);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -323,12 +299,11 @@ __global__ void __launch_bounds__(kNT, kCtasPerSm) k_solve_tc(SolveArgs<float> g
     ok = tc_wait(&mbar[(nst - 1) % kSets], uint32_t((nst - 1) / kSets) & 1u, g.status,
                  DCT_ERR_DEVICE_TIMEOUT, s, b);
   const float sgn = kInv ? 1.0f : -1.0f;
-  // rows 16-byte aligned and kc a multiple of 4: every output row of the
-  // tile goes out as one bulk reduction (cp.reduce.async.bulk .add.f32) from
-  // a staging copy in shared memory -- the operand buffers, free once the
-  // last MMA has completed -- instead of kc / 4 vector atomics per row.
-  const bool bulk = kTcBulkReduce && (g.k & 3) == 0;
-  if (ok && nst > 0 && bulk) {
+  // Every output row of the tile goes out as one bulk reduction
+  // (cp.reduce.async.bulk .add.f32) from a staging copy in shared memory --
+  // the operand buffers, free once the last MMA has completed -- instead of
+  // kc / 4 vector atomics per row.
+  if (ok && nst > 0) {
     float* stage = reinterpret_cast<float*>(smem_raw);
     // row stride: a multiple of 4 floats with stride / 4 odd, so that the
     // float4 stores of 8 consecutive rows hit distinct banks
@@ -370,33 +345,6 @@ __global__ void __launch_bounds__(kNT, kCtasPerSm) k_solve_tc(SolveArgs<float> g
       }
       __syncthreads();
     }
-  } else if (ok && nst > 0 && (warp & 3) * 32 < mvalid) {
-    const int m = (warp & 3) * 32 + lane;
-    float* dst = nullptr;
-    if (m < mvalid) {
-      const int64_t row = MODE == kModeFwdBnd ? int64_t(rows[ns + m0 + m])
-                                              : int64_t(first + m0 + m);
-      dst = Y + row * g.k + j0;
-    }
-    for (int cb = (warp >> 2) * 32; cb < np; cb += (kWarps / 4) * 32) {
-      uint32_t v[32];
-      tmem_ld32(tmem + (uint32_t((warp & 3) * 32) << 16) + uint32_t(cb), v);
-      if (dst != nullptr) {
-#pragma unroll
-        for (int c = 0; c < 32; c += 4) {
-          if (cb + c + 4 <= kc && (g.k & 3) == 0) {
-            atomicAdd(reinterpret_cast<float4*>(dst + cb + c),
-                      make_float4(sgn * __uint_as_float(v[c]), sgn * __uint_as_float(v[c + 1]),
-                                  sgn * __uint_as_float(v[c + 2]),
-                                  sgn * __uint_as_float(v[c + 3])));
-          } else {
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if (cb + c + q < kc) atomicAdd(dst + cb + c + q, sgn * __uint_as_float(v[c + q]));
-          }
-        }
-      }
-    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -407,6 +355,7 @@ __global__ void __launch_bounds__(kNT, kCtasPerSm) k_solve_tc(SolveArgs<float> g
 
 cudaError_t launch_solve_tc(int kind, const SolveArgs<float>& g0, int64_t count,
                             int nbatch, cudaStream_t st) {
+  if (g0.k % 4 != 0) return cudaErrorInvalidValue;
   SolveArgs<float> g = g0;
   g.nchunk = (g.k + kStN - 1) / kStN;
   dim3 grid(static_cast<unsigned>(count), static_cast<unsigned>(nbatch * g.nchunk));

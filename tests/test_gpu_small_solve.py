@@ -99,3 +99,20 @@ def test_long_boundary(cuda):
     gen = torch.Generator().manual_seed(3)
     check(slv, At, P, torch.randn(1, n, 9, dtype=torch.float64, generator=gen), cuda,
           4 * 8 * n * U[torch.float64])
+
+
+@pytest.mark.parametrize("shape", [(23, 14), (34, 33)])
+def test_refined_right_hand_side_counts(cuda, shape):
+    """Float32 plans with two corrections: rows of k right-hand sides that are and are not a
+    multiple of four (the work buffers pad them) and of two (16-byte rows).  With a condition
+    number below 4 the first correction already leaves less than (30 n_front u)^2, so what
+    remains is the rounding of the result: 2^-24, bounded here by twice that."""
+    P, crow, col, A = grid_system(shape, torch.float32, 2, 11)
+    n = P.shape[0]
+    slv = make_batch_solver(torch.tensor(crow), torch.tensor(col), n, 70, 2, device=cuda,
+                            dtype=torch.float32)
+    slv.factorize(A[:, torch.tensor(P)].to(cuda))
+    gen = torch.Generator().manual_seed(5)
+    for k in (1, 2, 3, 4, 5, 6, 7, 65, 66, 67, 68, 70):
+        check(slv, A, P, torch.randn(2, n, k, generator=gen), cuda, 2.0 ** -23)
+        check(slv, A, P, torch.randn(n, k, generator=gen), cuda, 2.0 ** -23)
