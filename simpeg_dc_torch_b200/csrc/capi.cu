@@ -197,7 +197,8 @@ dct_tuning resolve_tuning(int dtype, const dct_tuning* in) {
   // float64 fronts update after every panel (no blocking)
   if (in->update_block > 0 && dtype == DCT_F32) t.update_block = std::min(4, in->update_block);
   if (in->solve_target > 0) t.solve_target = in->solve_target;
-  if (in->solve_split_max > 0) t.solve_split_max = std::max(16, in->solve_split_max);
+  if (in->solve_split_max > 0)
+    t.solve_split_max = std::max(16, std::min(dct::kMaxSplitK, in->solve_split_max));
   if (in->solve_split_min > 0) t.solve_split_min = std::max(16, in->solve_split_min);
   t.solve_split_min = std::min(t.solve_split_min, t.solve_split_max);
   if (in->small_tc > 0) t.small_tc = std::min(2, in->small_tc);

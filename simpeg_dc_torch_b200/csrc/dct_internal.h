@@ -104,6 +104,9 @@ constexpr int kUpdateBlockPanels = DCT_UPDATE_BLOCK_PANELS;
 #endif
 constexpr int kUpdateBlockWide = DCT_UPDATE_BLOCK_WIDE;   // float64 and complex fronts
 
+// longest K piece of a float32 tensor-core substitution task
+constexpr int kMaxSplitK = 1024;
+
 // Column ranges of the trailing update that follows panel p of a supernode
 // with ns columns (front order N) when the panels are grouped in blocks of
 // bpan (LAPACK-style blocked right-looking Cholesky with an inner panel

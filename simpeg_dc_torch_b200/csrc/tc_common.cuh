@@ -142,6 +142,41 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, int* sta
   return done;
 }
 
+// one thread: bounded wait for phase `parity`
+__device__ __forceinline__ bool mbar_wait1(uint64_t* bar, uint32_t parity) {
+  for (uint32_t it = 0; it < kTcWaitLimit; ++it)
+    if (mbar_try_wait_sleep(smem_u32(bar), parity)) return true;
+  return false;
+}
+
+__device__ __forceinline__ void flag_timeout(int* status, int s, int b) {
+  if (atomicCAS(&status[0], 0, DCT_ERR_DEVICE_TIMEOUT) == 0) {
+    status[1] = s;
+    status[2] = b;
+  }
+}
+
+__device__ __forceinline__ void mbar_init_n(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+// one thread: bounded wait for phase `parity` that also gives up once another
+// role of the CTA has given up (*abort set); a timeout sets *abort
+__device__ __forceinline__ bool mbar_wait_ab(uint64_t* bar, uint32_t parity,
+                                             volatile int* abort) {
+  for (uint32_t it = 0; it < kTcWaitLimit; ++it) {
+    if (mbar_try_wait_sleep(smem_u32(bar), parity)) return true;
+    if (*abort) return false;
+  }
+  *abort = 1;
+  return false;
+}
+
 // 32 consecutive TMEM columns of this warp's 32 lanes (one row per thread)
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
