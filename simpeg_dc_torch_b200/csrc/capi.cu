@@ -600,6 +600,38 @@ void plan_persistent_updates(dct_plan* P) {
   }
 }
 
+// The column tasks and inverse row maps of k_large_assemble (factor.cu).
+int build_assembly(dct_plan* P) {
+  const dct::Symbolic& S = P->sym;
+  constexpr int kCols = dct::kThreads / 32;   // columns per task
+  std::vector<PanelTask> tasks;
+  std::vector<int32_t> inv;
+  std::vector<int64_t> off(S.nsuper, 0);
+  P->asm_first.assign(P->fact.launches.size(), 0);
+  P->asm_count.assign(P->fact.launches.size(), 0);
+  for (size_t li = 0; li < P->fact.launches.size(); ++li) {
+    const Launch& L = P->fact.launches[li];
+    if (L.kind != dct::kLargeScatter) continue;
+    P->asm_first[li] = int64_t(tasks.size());
+    for (int64_t q = L.first; q < L.first + L.count; ++q) {
+      const int s = P->fact.tasks[q].s, N = S.front_n[s];
+      for (int j = 0; j < N; j += kCols) tasks.push_back({s, j, 0, 0});
+      off[s] = int64_t(inv.size());
+      inv.resize(inv.size() + 2 * size_t(N), -1);
+      for (int u = 0; u < 2 && S.child_ptr[s] + u < S.child_ptr[s + 1]; ++u) {
+        const int c = S.child[S.child_ptr[s] + u];
+        for (int i = 0; i < S.nb(c); ++i)
+          inv[off[s] + int64_t(u) * N + S.rel[S.rel_ptr[c] + i]] = i;
+      }
+    }
+    P->asm_count[li] = int64_t(tasks.size()) - P->asm_first[li];
+  }
+  int rc = upload(P, inv, &P->d_inv);
+  if (rc == DCT_OK) rc = upload(P, off, &P->d_inv_off);
+  if (rc == DCT_OK) rc = upload(P, tasks, &P->d_asm);
+  return rc;
+}
+
 int upload_schedule(dct_plan* P, dct::Schedule* sch) {
   const PanelTask* d = nullptr;
   int rc = upload(P, sch->tasks, &d);
@@ -898,6 +930,7 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
       P->sm_count = sms;
   }
   plan_persistent_updates(P);
+  if ((rc = build_assembly(P))) return bail(rc);
   build_solve_schedules(S, dtype, P->tune, &P->fwd, &P->bwd);
   std::vector<int64_t> dinv_off;
   build_inverse_schedule(S, small_max, &P->inv, &dinv_off, &P->dinv_stride);

@@ -249,6 +249,12 @@ struct dct_plan {
   void* fronts = nullptr;          // nbatch * front_total elements of dtype
   int64_t front_stride = 0;
   dct::Schedule fact;              // factorization schedule
+  // assembly of the large fronts: inverse row maps of their first two children
+  // and, per factor launch of kind kLargeScatter, its column tasks
+  const int32_t* d_inv = nullptr;
+  const int64_t* d_inv_off = nullptr;
+  const dct::PanelTask* d_asm = nullptr;
+  std::vector<int64_t> asm_first, asm_count;
   dct::Schedule fwd;               // forward substitution schedule
   dct::Schedule bwd;               // backward substitution schedule
   dct::Schedule inv;               // diagonal-block inverses (one launch)

@@ -75,3 +75,16 @@ def test_one_wide_supernode(cuda, kind, nd):
     P[:3, 3:6] = P[3:6, :3] = False          # two small blocks only the dense one connects
     info = run(P, kind, cuda, (1, 7, 40, 66), nd, nbatch=1, leaf=4)
     assert info["max_ns"] > 160
+
+
+@pytest.mark.parametrize("kind", list(KINDS))
+@pytest.mark.parametrize("blocks,m,core", [(2, 30, 200), (3, 33, 230), (5, 20, 200), (7, 9, 300)])
+def test_front_with_many_children(cuda, kind, blocks, m, core):
+    """Dense blocks that only a dense core connects: one large front assembled from one, two or
+    more children (the first two in one pass, the others one by one)."""
+    n = blocks * m + core
+    P = np.zeros((n, n), bool)
+    for i in range(blocks):
+        P[i * m:(i + 1) * m, i * m:(i + 1) * m] = True
+    P[blocks * m:, :] = P[:, blocks * m:] = True
+    run(P, kind, cuda, (1, 20), blocks, nbatch=2, leaf=8)
