@@ -499,12 +499,11 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
   const int nb = P->nbatch;
   cudaError_t e = cudaSuccess;
   const int small_max = P->tune.small_front_max;
-  const size_t lu_smem = sizeof(T) * (size_t(small_max) * small_max + small_max);
+  const size_t lu_smem = small_lu_smem(small_max);
   const size_t panel_smem = sizeof(T) * (2 * kPanel * kPanelLd);
   // the update kernel's copy ring, or the diagonal block's workspace
-  constexpr int kDiagElems = kLuDiagElems > kBlockElems<T> ? kLuDiagElems : kBlockElems<T>;
-  constexpr int kUpdateElems = std::max(TilePipe<T, kUT, false>::kElems, kDiagElems);
-  const size_t update_smem = sizeof(T) * kUpdateElems;
+  const size_t update_smem =
+      sizeof(T) * std::max(TilePipe<T, kUT, false>::kElems, lu ? kLuDiagElems : kBlockElems<T>);
   // attributes are per device: set them on every call (cheap host calls)
   e = SmallLaunch<T, T>::allow(small_max);
   if constexpr (sizeof(T) == 4) {
@@ -538,8 +537,7 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
       case kSmallFront: {
         if constexpr (sizeof(T) == 8) {
           if (lu) {
-            const size_t smem = sizeof(T) * (size_t(L.arg) * L.arg + L.arg);
-            k_small_front_lu<<<grid, kThreads, smem, st>>>(
+            k_small_front_lu<<<grid, kThreads, small_lu_smem(L.arg), st>>>(
                 P->ds, t, static_cast<const double*>(vals), vals_stride, P->d_tr,
                 reinterpret_cast<double*>(fronts), reinterpret_cast<double*>(fronts2),
                 P->front_stride, P->status, P->pivot_floor);

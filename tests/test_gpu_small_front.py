@@ -102,3 +102,28 @@ def test_bad_pivot_is_reported_and_the_rest_is_solved(cuda, at):
     A[at, at] = 1.0
     ref = np.linalg.solve(A, b)
     assert np.linalg.norm(x - ref) <= 4 * n * 8 * n * 2.0 ** -53 * np.linalg.norm(ref)
+
+
+def test_general_front_of_every_edge_size(cuda):
+    """L U of one front (float64, rows and columns dominated by the diagonal: pivots grow by less
+    than 2 and the condition number stays below 4), A x = b and A^T x = b.  Tolerance as above,
+    doubled for the two factors."""
+    from simpeg_dc_torch_b200 import make_solver as make
+    for n in (m for m in SIZES if m <= 160):
+        rng = np.random.default_rng(n)
+        A = rng.uniform(-1, 1, (n, n))
+        np.fill_diagonal(A, 0.0)
+        A = A / max(1e-30, np.abs(A).sum(0).max(), np.abs(A).sum(1).max()) + 2.0 * np.eye(n)
+        b = rng.standard_normal((n, 3))
+        crow = np.arange(0, n * n + 1, n).astype(np.int32)
+        col = np.tile(np.arange(n), n).astype(np.int32)
+        slv = make(torch.tensor(crow), torch.tensor(col), n, 3, device=cuda,
+                   dtype=torch.float64, matrix_type="general", leaf_size=max(n, 1))
+        slv.factorize(torch.tensor(A.reshape(-1), device=cuda))
+        assert slv.static_pivots() == 0
+        for t in (False, True):
+            x = slv.solve(torch.tensor(b, device=cuda), transposed=t).cpu().numpy()
+            ref = np.linalg.solve(A.T if t else A, b)
+            err = np.linalg.norm(x - ref) / np.linalg.norm(ref)
+            assert err <= 4 * 16 * max(n, 4) * 2.0 ** -53, (n, t, err)
+        slv.check()
