@@ -657,6 +657,20 @@ int set_device(int device) {
 
 void dct::set_last_error(const char* msg) { g_err = msg; }
 
+cudaError_t dct::allow_smem(dct_plan* P, const void* kernel) {
+  for (const void* k : P->allowed)
+    if (k == kernel) return cudaSuccess;
+  int most = 0;
+  cudaFuncAttributes a;
+  cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, P->device);
+  if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kernel);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             most - static_cast<int>(a.sharedSizeBytes));
+  if (e == cudaSuccess) P->allowed.push_back(kernel);
+  return e;
+}
+
 cudaError_t dct::Profiler::begin(int kind, double flops, double bytes,
                                  cudaStream_t st) {
   if (!on) return cudaSuccess;

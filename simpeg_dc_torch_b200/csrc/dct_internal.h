@@ -288,6 +288,8 @@ struct dct_plan {
   // the number of diagonal tasks moved to the front of the launch's tasks
   // (one CTA each); -1: one CTA per task
   std::vector<int32_t> update_nspec;
+  // kernels whose dynamic shared memory limit this plan has raised
+  std::vector<const void*> allowed;
   dct::Profiler prof;
   // general (unsymmetric-valued) float64 plans, factored P A P^T = L U with
   // static pivoting: `fronts` holds L (unit diagonal) in the lower part,
@@ -328,9 +330,18 @@ struct SolveArgs {
   // the remaining correction solves return at entry (null: never skip)
   const int* skip;
 };
+// Raises a kernel's dynamic shared memory limit to all that the device has, the
+// first time the plan launches it.  The limit is one for the process and the
+// device, so it is the same for every plan: two threads that set it for the
+// sizes of their own launches would undo each other's.
+cudaError_t allow_smem(dct_plan* P, const void* kernel);
+template <typename... A>
+cudaError_t allow_smem(dct_plan* P, void (*kernel)(A...)) {
+  return allow_smem(P, reinterpret_cast<const void*>(kernel));
+}
 // one launch of a tensor-core substitution kind (kFwdLinvTc .. kBwdLinvTc)
-cudaError_t launch_solve_tc(int kind, const SolveArgs<float>& g, int64_t count,
-                            int nbatch, cudaStream_t st);
+cudaError_t launch_solve_tc(dct_plan* P, int kind, const SolveArgs<float>& g, int64_t count,
+                            cudaStream_t st);
 // one launch of the float32 trailing update (update_tc.cu); nspec >= 0:
 // the first nspec tasks take one CTA each and persistent CTAs on the
 // remaining multiprocessors share the others, nspec = -1: one CTA per task

@@ -427,12 +427,8 @@ cudaError_t run_linv(dct_plan* P, cudaStream_t st, const void* fronts, const voi
                      void* linv) {
   const int nb = P->nbatch;
   const size_t smem = sizeof(T) * TilePipe<T, kPanel, true>::kElems;
-  cudaError_t e = cudaFuncSetAttribute(k_linv_t<T>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_linv_x<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(smem));
+  cudaError_t e = allow_smem(P, k_linv_t<T>);
+  if (e == cudaSuccess) e = allow_smem(P, k_linv_x<T>);
   if (e != cudaSuccess) return e;
   LinvArgs g{P->ds, nullptr, P->front_stride, P->d_dinv_off, P->dinv_stride,
              P->d_linv_off, P->linv_stride, 0};
@@ -469,20 +465,12 @@ struct SmallLaunch {
   int64_t vals_stride;
   dim3 grid;
   cudaStream_t st;
-  static cudaError_t allow(int n) {
-    const cudaError_t e = cudaFuncSetAttribute(
-        k_small_front<T, G, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-        static_cast<int>(small_smem<T>(n)));
-    return e != cudaSuccess
-               ? e
-               : cudaFuncSetAttribute(k_small_front<T, G, kThreads / 2>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      static_cast<int>(small_smem<T>(std::min(kSmallNarrow, n))));
-  }
   cudaError_t operator()(int n) const {
     const bool narrow = n <= kSmallNarrow;
-    return launch_pdl(narrow ? k_small_front<T, G, kThreads / 2> : k_small_front<T, G, kThreads>,
-                      grid, dim3(narrow ? kThreads / 2 : kThreads), small_smem<T>(n), st, P->ds,
+    auto fn = narrow ? k_small_front<T, G, kThreads / 2> : k_small_front<T, G, kThreads>;
+    const cudaError_t e = allow_smem(P, fn);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(fn, grid, dim3(narrow ? kThreads / 2 : kThreads), small_smem<T>(n), st, P->ds,
                       tasks, vals, vals_dtype, vals_stride, static_cast<G*>(P->fronts),
                       P->front_stride, static_cast<G*>(P->dinv),
                       static_cast<const int64_t*>(P->d_dinv_off), P->dinv_stride, P->status);
@@ -498,30 +486,16 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
   T* fronts2 = lu ? static_cast<T*>(P->fronts2) : nullptr;
   const int nb = P->nbatch;
   cudaError_t e = cudaSuccess;
-  const int small_max = P->tune.small_front_max;
-  const size_t lu_smem = small_lu_smem(small_max);
   const size_t panel_smem = sizeof(T) * (2 * kPanel * kPanelLd);
   // the update kernel's copy ring, or the diagonal block's workspace
   const size_t update_smem =
       sizeof(T) * std::max(TilePipe<T, kUT, false>::kElems, lu ? kLuDiagElems : kBlockElems<T>);
-  // attributes are per device: set them on every call (cheap host calls)
-  e = SmallLaunch<T, T>::allow(small_max);
-  if constexpr (sizeof(T) == 4) {
-    if (e == cudaSuccess) e = SmallLaunch<double, T>::allow(std::min(small_max, kSmallFrontF64));
-  }
   if constexpr (sizeof(T) == 8) {
-    if (e == cudaSuccess && lu)
-      e = cudaFuncSetAttribute(k_small_front_lu, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(lu_smem));
+    if (lu) e = allow_smem(P, k_small_front_lu);
   }
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_large_panel<T>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(panel_smem));
+  if (e == cudaSuccess) e = allow_smem(P, k_large_panel<T>);
   if constexpr (sizeof(T) != 4) {
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k_large_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(update_smem));
+    if (e == cudaSuccess) e = allow_smem(P, k_large_update<T>);
   }
   if (e != cudaSuccess) return e;
   const PanelTask* tasks = P->fact.d_tasks;
@@ -611,8 +585,7 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
     const int64_t ninv = int64_t(P->inv.tasks.size());
     if (lu && ninv > 0) {
       const size_t inv_smem = sizeof(T) * kBlockElems<T>;
-      e = cudaFuncSetAttribute(k_panel_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               static_cast<int>(inv_smem));
+      e = allow_smem(P, k_panel_inverse);
       if (e == cudaSuccess) e = P->prof.begin(kPanelInverse, 0.0, 0.0, st);
       if (e != cudaSuccess) return e;
       const dim3 grid(static_cast<unsigned>(ninv), nb);

@@ -412,13 +412,12 @@ int tile_columns(int k) { return k <= 8 ? 8 : (k <= 16 ? 16 : (k <= 32 ? 32 : 64
 
 // one launch of a substitution kind on tiles of NC right-hand sides
 template <typename T, int NC>
-cudaError_t launch_tiles(int kind, SolveArgs<T> g, const SmallShape& sh, int64_t count, int nbatch,
-                         cudaStream_t st) {
+cudaError_t launch_tiles(dct_plan* P, int kind, SolveArgs<T> g, const SmallShape& sh,
+                         int64_t count, cudaStream_t st) {
   g.nchunk = (g.k + NC - 1) / NC;
-  const dim3 grid(static_cast<unsigned>(count * g.nchunk), nbatch), block(kThreads);
+  const dim3 grid(static_cast<unsigned>(count * g.nchunk), P->nbatch), block(kThreads);
   auto go = [&](auto fn, size_t smem, auto... more) {
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+    const cudaError_t e = allow_smem(P, fn);
     return e != cudaSuccess ? e : launch_pdl(fn, grid, block, smem, st, g, more...);
   };
   if (kind == kFwdSmall || kind == kBwdSmall) {
@@ -442,16 +441,16 @@ cudaError_t launch_tiles(int kind, SolveArgs<T> g, const SmallShape& sh, int64_t
   return cudaErrorInvalidValue;
 }
 template <typename T>
-cudaError_t launch_tiles(int kind, const SolveArgs<T>& g, SmallShape sh, int64_t count, int nbatch,
-                         cudaStream_t st) {
+cudaError_t launch_tiles(dct_plan* P, int kind, const SolveArgs<T>& g, SmallShape sh,
+                         int64_t count, cudaStream_t st) {
   constexpr int V = 16 / sizeof(T);
   sh.wide = g.k % V == 0 && (reinterpret_cast<uintptr_t>(g.A) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(g.B) & 15) == 0;
   switch (tile_columns(g.k)) {
-    case 8: return launch_tiles<T, 8>(kind, g, sh, count, nbatch, st);
-    case 16: return launch_tiles<T, 16>(kind, g, sh, count, nbatch, st);
-    case 32: return launch_tiles<T, 32>(kind, g, sh, count, nbatch, st);
-    default: return launch_tiles<T, 64>(kind, g, sh, count, nbatch, st);
+    case 8: return launch_tiles<T, 8>(P, kind, g, sh, count, st);
+    case 16: return launch_tiles<T, 16>(P, kind, g, sh, count, st);
+    case 32: return launch_tiles<T, 32>(P, kind, g, sh, count, st);
+    default: return launch_tiles<T, 64>(P, kind, g, sh, count, st);
   }
 }
 
@@ -516,16 +515,16 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
         case kBwdGemmTc:
         case kBwdLinvTc:
           if constexpr (kTc) {
-            e = launch_solve_tc(L.kind, g, L.count, P->nbatch, st);
+            e = launch_solve_tc(P, L.kind, g, L.count, st);
             if (e != cudaSuccess) return e;
             break;
           }
           return cudaErrorInvalidValue;
         default:
           // every launch of a solve but the first follows one of its own
-          e = launch_tiles<T>(L.kind, g, SmallShape{sc->max_ns[li], sc->max_nb[li],
-                                                    pass == 1 || li > 0, 0},
-                              L.count, P->nbatch, st);
+          e = launch_tiles<T>(P, L.kind, g, SmallShape{sc->max_ns[li], sc->max_nb[li],
+                                                       pass == 1 || li > 0, 0},
+                              L.count, st);
           if (e != cudaSuccess) return e;
       }
       if ((e = cudaGetLastError()) != cudaSuccess) return e;

@@ -339,28 +339,22 @@ __global__ void __launch_bounds__(kTcCta, kCtasPerSm) k_solve_tc(SolveArgs<float
 
 }  // namespace
 
-cudaError_t launch_solve_tc(int kind, const SolveArgs<float>& g0, int64_t count,
-                            int nbatch, cudaStream_t st) {
+cudaError_t launch_solve_tc(dct_plan* P, int kind, const SolveArgs<float>& g0, int64_t count,
+                            cudaStream_t st) {
   if (g0.k % 4 != 0) return cudaErrorInvalidValue;
   SolveArgs<float> g = g0;
   g.nchunk = (g.k + kStN - 1) / kStN;
-  dim3 grid(static_cast<unsigned>(count), static_cast<unsigned>(nbatch * g.nchunk));
-  const void* fn = nullptr;
+  const dim3 grid(static_cast<unsigned>(count), static_cast<unsigned>(P->nbatch * g.nchunk));
+  auto go = [&](auto fn) {
+    const cudaError_t e = allow_smem(P, fn);
+    return e != cudaSuccess ? e : launch_pdl(fn, grid, dim3(kTcCta), kSolveTcSmem, st, g);
+  };
   switch (kind) {
-    case kFwdLinvTc: fn = reinterpret_cast<const void*>(k_solve_tc<kModeFwdLinv>); break;
-    case kFwdBndTc: fn = reinterpret_cast<const void*>(k_solve_tc<kModeFwdBnd>); break;
-    case kBwdGemmTc: fn = reinterpret_cast<const void*>(k_solve_tc<kModeBwdGemm>); break;
-    case kBwdLinvTc: fn = reinterpret_cast<const void*>(k_solve_tc<kModeBwdLinv>); break;
+    case kFwdLinvTc: return go(k_solve_tc<kModeFwdLinv>);
+    case kFwdBndTc: return go(k_solve_tc<kModeFwdBnd>);
+    case kBwdGemmTc: return go(k_solve_tc<kModeBwdGemm>);
+    case kBwdLinvTc: return go(k_solve_tc<kModeBwdLinv>);
     default: return cudaErrorInvalidValue;
-  }
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(kSolveTcSmem));
-  if (e != cudaSuccess) return e;
-  switch (kind) {
-    case kFwdLinvTc: return launch_pdl(k_solve_tc<kModeFwdLinv>, grid, dim3(kTcCta), kSolveTcSmem, st, g);
-    case kFwdBndTc: return launch_pdl(k_solve_tc<kModeFwdBnd>, grid, dim3(kTcCta), kSolveTcSmem, st, g);
-    case kBwdGemmTc: return launch_pdl(k_solve_tc<kModeBwdGemm>, grid, dim3(kTcCta), kSolveTcSmem, st, g);
-    default: return launch_pdl(k_solve_tc<kModeBwdLinv>, grid, dim3(kTcCta), kSolveTcSmem, st, g);
   }
 }
 

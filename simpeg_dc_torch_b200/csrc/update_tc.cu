@@ -502,8 +502,7 @@ k_update_tc(DevSym S, const PanelTask* __restrict__ tasks, float* fronts,
 
 cudaError_t launch_update_tc(dct_plan* P, const PanelTask* tasks, int64_t count, int nspec,
                              cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(k_update_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(kUSmem));
+  const cudaError_t e = allow_smem(P, k_update_tc);
   if (e != cudaSuccess) return e;
   dim3 grid(static_cast<unsigned>(count), static_cast<unsigned>(P->nbatch));
   if (nspec >= 0) {
