@@ -988,6 +988,21 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
   }
   account_factor(S, &P->fact, double(esize(dtype)), update_tile(dtype),
                  P->update_bpan, dtype == DCT_F32);
+  // the marks of the supernodes that a right-hand side reaches serve the large
+  // forward products only (the single-panel ones look at their own rows)
+  bool marks = false;
+  for (const dct::Launch& L : P->fwd.launches)
+    marks = marks || (L.count > 0 && L.kind != dct::kFwdSmall);
+  if (marks && dtype != DCT_C128 && !P->lu) {
+    std::vector<int32_t> sn_of(S.n);
+    for (int s = 0; s < S.nsuper; ++s)
+      for (int i = S.sn_first[s]; i < S.sn_first[s + 1]; ++i) sn_of[i] = s;
+    void* d = nullptr;
+    if ((rc = upload(P, sn_of, &P->d_sn_of)) || (rc = upload(P, S.sn_parent, &P->d_parent)) ||
+        (rc = alloc(P, sizeof(int32_t) * size_t(nbatch) * S.nsuper, &d, "supernode marks")))
+      return bail(rc);
+    P->nz = static_cast<int32_t*>(d);
+  }
   if (dtype == DCT_F32) {
     // the supernodes without a single-panel task
     std::vector<char> small(S.nsuper, 0);
@@ -1177,8 +1192,8 @@ int solve_refined(dct_plan* P, const double* bp, int64_t bstride, int k,
                   double* xp, cudaStream_t st) {
   DCT_CUDA(cudaMemsetAsync(P->resid_bits, 0, 16, st), "memset");
   DCT_CUDA(cudaMemsetAsync(P->ir, 0, sizeof(dct::IrState), st), "memset");
-  DCT_CUDA(dct::launch_rhs_to_float(P, bp, bstride, k, st), "rhs conversion");
-  DCT_CUDA(dct::run_solve_f32(P, k, st), "solve launch");
+  DCT_CUDA(dct::launch_rhs_in(P, bp, bstride, k, P->bufA, st), "rhs conversion");
+  DCT_CUDA(dct::run_solve_f32(P, k, st, true), "solve launch");
   DCT_CUDA(dct::launch_ir_update(P, xp, k, 1, st), "refinement update");
   // corrections until the estimated error is below the tolerance, the
   // iterations stagnate or ir_iters are spent; the decision is taken on the
@@ -1211,11 +1226,9 @@ int dct_solve_permuted(dct_plan* P, const double* d_bp, int32_t b_batched,
   const int64_t per = int64_t(P->sym.n) * k;
   const int64_t bstride = b_batched ? per : 0;
   if (P->dtype == DCT_F64) {
-    if (d_bp != d_xp || !b_batched)
-      DCT_CUDA(dct::launch_convert_any(d_bp, DCT_F64, bstride, per, P->nbatch,
-                                       d_xp, DCT_F64, st),
-               "rhs copy");
-    DCT_CUDA(dct::run_solve_f64(P, d_xp, k, st), "solve launch");
+    const bool copy = d_bp != d_xp || !b_batched;
+    if (copy) DCT_CUDA(dct::launch_rhs_in(P, d_bp, bstride, k, d_xp, st), "rhs copy");
+    DCT_CUDA(dct::run_solve_f64(P, d_xp, k, st, false, copy), "solve launch");
     return DCT_OK;
   }
   return solve_refined(P, d_bp, bstride, k, d_xp, st);

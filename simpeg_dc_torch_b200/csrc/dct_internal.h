@@ -275,6 +275,9 @@ struct dct_plan {
   unsigned long long* resid_bits = nullptr;  // device: max|r|, max|b|
   int factored = 0;
   int64_t stamp = 0;
+  const int32_t* d_sn_of = nullptr;   // supernode of each row (permuted order)
+  const int32_t* d_parent = nullptr;  // parent supernode, -1: a root
+  int32_t* nz = nullptr;              // nbatch * nsuper marks of a solve (launch_rhs_in)
   const int32_t* d_tc = nullptr;   // f32 plans: supernodes solved by the tensor-core
   int32_t n_tc = 0;                //   products, and how many they are
   dct::ImgArgs img{};              // f32 plans: split panel images (large fronts)
@@ -329,7 +332,15 @@ struct SolveArgs {
   // float32 plans: refinement state; a set `done` word makes every kernel of
   // the remaining correction solves return at entry (null: never skip)
   const int* skip;
+  // forward pass: the supernodes (of each system) that the right-hand sides
+  // reach, nsuper marks per system (null: all of them)
+  const int32_t* nz;
+  int nsuper;
 };
+template <typename T>
+__device__ __forceinline__ bool rhs_reaches(const SolveArgs<T>& g, int s, int b) {
+  return g.nz == nullptr || g.nz[int64_t(b) * g.nsuper + s] != 0;
+}
 // Raises a kernel's dynamic shared memory limit to all that the device has, the
 // first time the plan launches it.  The limit is one for the process and the
 // device, so it is the same for every plan: two threads that set it for the
@@ -352,8 +363,8 @@ void set_last_error(const char* msg);
 cudaError_t run_factor(dct_plan* P, const void* vals, int vals_dtype,
                        int64_t vals_stride, cudaStream_t st);
 cudaError_t run_solve_f64(dct_plan* P, double* xa, int k, cudaStream_t st,
-                          bool transposed = false);
-cudaError_t run_solve_f32(dct_plan* P, int k, cudaStream_t st);
+                          bool transposed = false, bool marked = false);
+cudaError_t run_solve_f32(dct_plan* P, int k, cudaStream_t st, bool marked = false);
 // complex128 plans: the permuted right-hand side in xa (solution left there)
 cudaError_t run_solve_c128(dct_plan* P, cplx* xa, int k, cudaStream_t st);
 cudaError_t launch_perm_in_any(const void* b, int b_dtype, int64_t bstride,
@@ -367,9 +378,10 @@ cudaError_t launch_convert_any(const void* src, int src_dtype, int64_t sstride,
                                int dst_dtype, cudaStream_t st);
 // floats in a row of the float32 plans' right-hand sides (see solve.cu)
 inline int rhs_ld(int k) { return (k + 3) & ~3; }
-// b (float64, permuted) -> buffer A of a float32 plan
-cudaError_t launch_rhs_to_float(dct_plan* P, const double* b, int64_t bstride, int k,
-                                cudaStream_t st);
+// b (float64, permuted) -> the right-hand sides of a float32 or float64 solve,
+// marking the supernodes that they reach
+cudaError_t launch_rhs_in(dct_plan* P, const double* b, int64_t bstride, int k, void* rhs,
+                          cudaStream_t st);
 cudaError_t launch_residual(dct_plan* P, const double* b, int64_t bstride,
                             const double* x, int k, cudaStream_t st);
 cudaError_t launch_ir_update(dct_plan* P, double* x, int k, int first,

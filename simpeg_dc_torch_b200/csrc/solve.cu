@@ -60,6 +60,12 @@ __global__ void __launch_bounds__(kThreads, kLargeCtas<T>) k_fwd_linv(SolveArgs<
   pdl_trigger();
   SmallTile<T, NC> acc;
   acc.zero();
+  if (!rhs_reaches(g, s, b)) {   // y = 0
+    acc.each(nr, [&](int r, int j, T& v) {
+      if (r < nr && j < rc) Bo[int64_t(first + r0 + r) * g.k + j0 + j] = v;
+    });
+    return;
+  }
   ColStream<T, kPanel> a(X + r0, ns, nr);
   RhsStream<T, NC, V, false> x(A, g.k, j0, rc, first, nullptr);
   TilePipe<T, NC, false>::run(reinterpret_cast<T*>(smem_raw), r0 + nr, nr, rc, acc, a, x);
@@ -116,6 +122,7 @@ __global__ void __launch_bounds__(kThreads, kLargeCtas<T>) k_fwd_bnd(SolveArgs<T
   const T* Bo = g.B + int64_t(b) * g.n * g.k;
   pdl_wait();
   pdl_trigger();
+  if (!rhs_reaches(g, s, b)) return;
   SmallTile<T, NC> acc;
   acc.zero();
   ColStream<T, kPanel> a(F + r0, N, nr);
@@ -228,21 +235,44 @@ __device__ __forceinline__ void load_quad(const double* p, int left, double (&v)
   }
 }
 
-// b (float64, n x k) -> the float32 right-hand sides
-template <int V>
-__global__ void k_rhs_to_float(const double* __restrict__ b, int64_t bstride, int n, int k, int kp,
-                               float* __restrict__ r32) {
-  const int kq = kp / 4;
+// b (float64, n x k) -> buffer A of a solve: float rows of kp for float32 plans,
+// double rows of kp = k for float64 ones.  nz (null: not wanted) marks, for each
+// system, the supernodes that a nonzero row belongs to (sn_of) and those above
+// them: the sources of a survey are a few electrodes, and the large forward
+// products of every other supernode have nothing to do.  A walk upwards ends
+// at a mark: whoever set that one walks on from it.
+template <typename T, int V>
+__global__ void k_rhs_in(const double* __restrict__ b, int64_t bstride, int n, int k, int kp,
+                         T* __restrict__ rhs, const int32_t* __restrict__ sn_of,
+                         const int32_t* __restrict__ parent, int32_t* nz, int nsuper) {
+  const int kq = kp / 4 + (kp % 4 != 0);
   const int64_t total = int64_t(n) * kq;
   const double* Bv = b + int64_t(blockIdx.y) * bstride;
-  float4* R = reinterpret_cast<float4*>(r32) + int64_t(blockIdx.y) * total;
+  T* R = rhs + int64_t(blockIdx.y) * n * kp;
+  volatile int32_t* mark = nz + (nz != nullptr ? int64_t(blockIdx.y) * nsuper : 0);
   for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
        idx += int64_t(gridDim.x) * blockDim.x) {
     const int64_t i = idx / kq;
-    const int j = static_cast<int>(idx - i * kq) * 4;
+    const int j = static_cast<int>(idx - i * kq) * 4, left = k - j;
     double v[4];
-    load_quad<V>(Bv + i * k + j, k - j, v);
-    R[idx] = make_float4(float(v[0]), float(v[1]), float(v[2]), float(v[3]));
+    load_quad<V>(Bv + i * k + j, left, v);
+    T* r = R + i * kp + j;
+    if constexpr (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(r) =
+          make_float4(float(v[0]), float(v[1]), float(v[2]), float(v[3]));
+    } else {
+#pragma unroll
+      for (int h = 0; h < 4; h += V)
+        if (h < left) {
+          if constexpr (V == 2)
+            *reinterpret_cast<double2*>(r + h) = make_double2(v[h], v[h + 1]);
+          else
+            r[h] = v[h];
+        }
+    }
+    // (a NaN is not a zero)
+    if (nz != nullptr && !(v[0] == 0.0 && v[1] == 0.0 && v[2] == 0.0 && v[3] == 0.0))
+      for (int s = sn_of[i]; s >= 0 && mark[s] == 0; s = parent[s]) mark[s] = 1;
   }
 }
 
@@ -464,13 +494,14 @@ inline dim3 grid1d(int64_t total, int ny) {
 // M = U^T, so the forward pass runs on M and the backward pass on L)
 template <typename T>
 cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
-                       bool transposed = false) {
+                       bool transposed = false, bool marked = false) {
   cudaError_t e = cudaSuccess;
   SolveArgs<T> g{P->ds, nullptr, static_cast<const T*>(P->fronts), P->front_stride,
                  static_cast<const T*>(P->dinv), P->d_dinv_off, P->dinv_stride,
                  bufA, bufB, P->sym.n, k, 1, P->status,
                  static_cast<const T*>(P->linv), P->d_linv_off, P->linv_stride,
-                 P->dtype == DCT_F32 && P->ir != nullptr ? &P->ir->done : nullptr};
+                 P->dtype == DCT_F32 && P->ir != nullptr ? &P->ir->done : nullptr,
+                 marked ? P->nz : nullptr, P->sym.nsuper};
   constexpr bool kTc = sizeof(T) == 4;
   const size_t work = sizeof(T) * size_t(P->nbatch) * P->sym.n * k;
   const double nb = P->nbatch;
@@ -537,10 +568,11 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
 }  // namespace
 
 // f64 plans: the permuted right-hand side is in `xa` (buffer A) and the
-// solution is left there; P->bufB serves as buffer B.
+// solution is left there; P->bufB serves as buffer B.  marked: launch_rhs_in
+// marked the supernodes that its rows reach.
 cudaError_t run_solve_f64(dct_plan* P, double* xa, int k, cudaStream_t st,
-                          bool transposed) {
-  return solve_impl<double>(P, xa, static_cast<double*>(P->bufB), k, st, transposed);
+                          bool transposed, bool marked) {
+  return solve_impl<double>(P, xa, static_cast<double*>(P->bufB), k, st, transposed, marked);
 }
 
 // complex128 plans: as float64, on complex buffers
@@ -550,9 +582,9 @@ cudaError_t run_solve_c128(dct_plan* P, cplx* xa, int k, cudaStream_t st) {
 
 // f32 plans: right-hand side in P->bufA (float, A), P->bufB (B), rows of
 // rhs_ld(k).
-cudaError_t run_solve_f32(dct_plan* P, int k, cudaStream_t st) {
+cudaError_t run_solve_f32(dct_plan* P, int k, cudaStream_t st, bool marked) {
   return solve_impl<float>(P, static_cast<float*>(P->bufA), static_cast<float*>(P->bufB),
-                           rhs_ld(k), st);
+                           rhs_ld(k), st, false, marked);
 }
 
 cudaError_t launch_perm_in_any(const void* b, int b_dtype, int64_t bstride,
@@ -629,12 +661,28 @@ static bool even_rows(const double* p, int64_t stride, int k) {
   return k % 2 == 0 && stride % 2 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
 }
 
-cudaError_t launch_rhs_to_float(dct_plan* P, const double* b, int64_t bstride, int k,
-                                cudaStream_t st) {
-  const int n = P->sym.n, kp = rhs_ld(k);
-  auto fn = even_rows(b, bstride, k) ? k_rhs_to_float<2> : k_rhs_to_float<1>;
-  fn<<<grid1d(int64_t(n) * kp / 4, P->nbatch), kThreads, 0, st>>>(b, bstride, n, k, kp,
-                                                                 static_cast<float*>(P->bufA));
+cudaError_t launch_rhs_in(dct_plan* P, const double* b, int64_t bstride, int k, void* rhs,
+                          cudaStream_t st) {
+  const int n = P->sym.n, nsuper = P->sym.nsuper;
+  const bool f32 = P->dtype == DCT_F32;
+  const int kp = f32 ? rhs_ld(k) : k;
+  if (P->nz != nullptr) {
+    const cudaError_t e =
+        cudaMemsetAsync(P->nz, 0, sizeof(int32_t) * size_t(P->nbatch) * nsuper, st);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 g = grid1d(int64_t(n) * ((kp + 3) / 4), P->nbatch);
+  // the copies of the float64 rows are as wide as both sides allow
+  const bool even = even_rows(b, bstride, k) &&
+                    (f32 || (reinterpret_cast<uintptr_t>(rhs) & 15) == 0);
+  auto go = [&](auto* out, auto fn) {
+    fn<<<g, kThreads, 0, st>>>(b, bstride, n, k, kp, out, P->d_sn_of, P->d_parent, P->nz,
+                               nsuper);
+  };
+  if (f32)
+    go(static_cast<float*>(rhs), even ? k_rhs_in<float, 2> : k_rhs_in<float, 1>);
+  else
+    go(static_cast<double*>(rhs), even ? k_rhs_in<double, 2> : k_rhs_in<double, 1>);
   return cudaGetLastError();
 }
 

@@ -150,7 +150,10 @@ __global__ void __launch_bounds__(kTcCta, kCtasPerSm) k_solve_tc(SolveArgs<float
   pdl_trigger();
   const uint32_t idesc = umma_idesc_tf32(kTcM, np);
   // a finished refinement: the remaining correction launches do nothing
-  const bool skip = g.skip != nullptr && *reinterpret_cast<const volatile int*>(g.skip) != 0;
+  bool skip = g.skip != nullptr && *reinterpret_cast<const volatile int*>(g.skip) != 0;
+  // nor does the forward pass for a supernode without right-hand sides (its
+  // rows of B are cleared)
+  if constexpr (!kTrans) skip = skip || !rhs_reaches(g, s, b);
   const int nst = skip ? 0 : (k1 - k0 + kStK - 1) / kStK;
   // This thread's values of a stage.  Natural A: row m = tid % 128, K quads
   // tid / 128 and + 2 (a warp's loads are 32 consecutive rows); transposed A:
