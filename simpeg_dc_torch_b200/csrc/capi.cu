@@ -988,21 +988,6 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
   }
   account_factor(S, &P->fact, double(esize(dtype)), update_tile(dtype),
                  P->update_bpan, dtype == DCT_F32);
-  // the marks of the supernodes that a right-hand side reaches serve the large
-  // forward products only (the single-panel ones look at their own rows)
-  bool marks = false;
-  for (const dct::Launch& L : P->fwd.launches)
-    marks = marks || (L.count > 0 && L.kind != dct::kFwdSmall);
-  if (marks && dtype != DCT_C128 && !P->lu) {
-    std::vector<int32_t> sn_of(S.n);
-    for (int s = 0; s < S.nsuper; ++s)
-      for (int i = S.sn_first[s]; i < S.sn_first[s + 1]; ++i) sn_of[i] = s;
-    void* d = nullptr;
-    if ((rc = upload(P, sn_of, &P->d_sn_of)) || (rc = upload(P, S.sn_parent, &P->d_parent)) ||
-        (rc = alloc(P, sizeof(int32_t) * size_t(nbatch) * S.nsuper, &d, "supernode marks")))
-      return bail(rc);
-    P->nz = static_cast<int32_t*>(d);
-  }
   if (dtype == DCT_F32) {
     // the supernodes without a single-panel task
     std::vector<char> small(S.nsuper, 0);
@@ -1017,6 +1002,27 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
   }
   account_solve(S, &P->fwd, double(esize(dtype)));
   account_solve(S, &P->bwd, double(esize(dtype)));
+  // the marks of the supernodes that a right-hand side reaches serve the large
+  // forward products (the single-panel ones look at their own rows), so plans
+  // that spend less than half of the forward pass there go without: in 2-D
+  // grids the marks cost as much as they save (56 us a solve against 27 without
+  // and 20 us of products, line of 38 sources)
+  double large = 0, all = 0;
+  for (size_t i = 0; i < P->fwd.launches.size(); ++i) {
+    all += P->fwd.flops[i];
+    if (P->fwd.launches[i].kind != dct::kFwdSmall) large += P->fwd.flops[i];
+  }
+  const bool marks = large >= 0.5 * all && large > 0;
+  if (marks && dtype != DCT_C128 && !P->lu) {
+    std::vector<int32_t> sn_of(S.n);
+    for (int s = 0; s < S.nsuper; ++s)
+      for (int i = S.sn_first[s]; i < S.sn_first[s + 1]; ++i) sn_of[i] = s;
+    void* d = nullptr;
+    if ((rc = upload(P, sn_of, &P->d_sn_of)) || (rc = upload(P, S.sn_parent, &P->d_parent)) ||
+        (rc = alloc(P, sizeof(int32_t) * size_t(nbatch) * S.nsuper, &d, "supernode marks")))
+      return bail(rc);
+    P->nz = static_cast<int32_t*>(d);
+  }
   if ((rc = upload_schedule(P, &P->fact)) || (rc = upload_schedule(P, &P->fwd)) ||
       (rc = upload_schedule(P, &P->bwd)) || (rc = upload_schedule(P, &P->inv)) ||
       (rc = upload_schedule(P, &P->linv_sched)))
