@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "dct_internal.h"
 #include "solve_small.cuh"
@@ -436,23 +437,34 @@ __global__ void k_ir_decide(IrState* ir, int* status, unsigned long long* resid_
   }
 }
 
-// right-hand sides per CTA of the kernels above: the fewest columns that hold
+// right-hand sides per CTA of the products of the larger supernodes: the fewest columns that hold
 // k, or chunks of 64 (whose fragments beyond k the double products skip)
 int tile_columns(int k) { return k <= 8 ? 8 : (k <= 16 ? 16 : (k <= 32 ? 32 : 64)); }
 
 // one launch of a substitution kind on tiles of NC right-hand sides
 template <typename T, int NC>
-cudaError_t launch_tiles(dct_plan* P, int kind, SolveArgs<T> g, const SmallShape& sh,
+cudaError_t launch_tiles(dct_plan* P, int kind, SolveArgs<T> g, SmallShape sh,
                          int64_t count, cudaStream_t st) {
   g.nchunk = (g.k + NC - 1) / NC;
-  const dim3 grid(static_cast<unsigned>(count * g.nchunk), P->nbatch), block(kThreads);
+  dim3 grid(static_cast<unsigned>(count * g.nchunk), P->nbatch);
+  const dim3 block(kThreads);
   auto go = [&](auto fn, size_t smem, auto... more) {
     const cudaError_t e = allow_smem(P, fn);
     return e != cudaSuccess ? e : launch_pdl(fn, grid, block, smem, st, g, more...);
   };
   if (kind == kFwdSmall || kind == kBwdSmall) {
-    const size_t smem = SmallPlaces<T, NC>(sh.w, sh.nb).bytes(sh.nb);
-    return kind == kFwdSmall ? go(k_fwd_small<T, NC>, smem, sh) : go(k_bwd_small<T, NC>, smem, sh);
+    sh.chunks = small_chunks<T, NC>(count * P->nbatch, sh.nb, g.nchunk);
+    grid.x = static_cast<unsigned>(count * ((g.nchunk + sh.chunks - 1) / sh.chunks));
+    const int in = kind == kFwdSmall ? sh.w : std::min(sh.nb, kPanel);
+    const size_t smem = SmallPlaces<T, NC>(sh.w, sh.nb, in, sh.chunks > 1).bytes(sh.nb);
+    auto small = [&](auto loop) {
+      constexpr bool L = decltype(loop)::value;
+      return kind == kFwdSmall ? go(k_fwd_small<T, NC, L>, smem, sh)
+                               : go(k_bwd_small<T, NC, L>, smem, sh);
+    };
+    if constexpr (kSmallLoop<T, NC>)
+      if (sh.chunks > 1) return small(std::true_type{});
+    return small(std::false_type{});
   }
   if constexpr (sizeof(T) != 4) {
     constexpr size_t km = sizeof(T) * TilePipe<T, NC, false>::kElems;
@@ -476,7 +488,8 @@ cudaError_t launch_tiles(dct_plan* P, int kind, const SolveArgs<T>& g, SmallShap
   constexpr int V = 16 / sizeof(T);
   sh.wide = g.k % V == 0 && (reinterpret_cast<uintptr_t>(g.A) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(g.B) & 15) == 0;
-  switch (tile_columns(g.k)) {
+  const bool small = kind == kFwdSmall || kind == kBwdSmall;
+  switch (small ? small_columns<T>(g.k, sh.w, sh.nb) : tile_columns(g.k)) {
     case 8: return launch_tiles<T, 8>(P, kind, g, sh, count, st);
     case 16: return launch_tiles<T, 16>(P, kind, g, sh, count, st);
     case 32: return launch_tiles<T, 32>(P, kind, g, sh, count, st);
@@ -554,7 +567,7 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
         default:
           // every launch of a solve but the first follows one of its own
           e = launch_tiles<T>(P, L.kind, g, SmallShape{sc->max_ns[li], sc->max_nb[li],
-                                                       pass == 1 || li > 0, 0},
+                                                       pass == 1 || li > 0, 0, 1},
                               L.count, st);
           if (e != cudaSuccess) return e;
       }
