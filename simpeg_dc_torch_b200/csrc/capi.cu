@@ -1022,6 +1022,23 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
         (rc = alloc(P, sizeof(int32_t) * size_t(nbatch) * S.nsuper, &d, "supernode marks")))
       return bail(rc);
     P->nz = static_cast<int32_t*>(d);
+  } else if (dtype == DCT_F64 && !P->fwd.launches.empty() &&
+             P->fwd.launches[0].kind == dct::kFwdSmall && P->fwd.launches[0].level == 0) {
+    // Leaves have three quarters of the rows of a 2-D grid, and no boundary
+    // update reaches them: they take their right-hand sides from the caller's
+    // array, mostly one array for all systems, instead of a copy per system.
+    // Measured on a B200, the copies of two solves: 610 -> 129 us on the
+    // 56,525-node line (12 systems, 186 sources), 251 -> 59 us on ten lines of
+    // 72 sources.
+    const Launch& l = P->fwd.launches[0];
+    std::vector<char> leaf(S.nsuper, 0);
+    for (int64_t q = l.first; q < l.first + l.count; ++q) leaf[P->fwd.tasks[q].s] = 1;
+    std::vector<int32_t> inner;
+    for (int s = 0; s < S.nsuper; ++s)
+      for (int i = S.sn_first[s]; !leaf[s] && i < S.sn_first[s + 1]; ++i) inner.push_back(i);
+    P->n_inner = static_cast<int32_t>(inner.size());
+    if (inner.empty()) inner.push_back(0);
+    if ((rc = upload(P, inner, &P->d_inner))) return bail(rc);
   }
   if ((rc = upload_schedule(P, &P->fact)) || (rc = upload_schedule(P, &P->fwd)) ||
       (rc = upload_schedule(P, &P->bwd)) || (rc = upload_schedule(P, &P->inv)) ||
@@ -1234,7 +1251,8 @@ int dct_solve_permuted(dct_plan* P, const double* d_bp, int32_t b_batched,
   if (P->dtype == DCT_F64) {
     const bool copy = d_bp != d_xp || !b_batched;
     if (copy) DCT_CUDA(dct::launch_rhs_in(P, d_bp, bstride, k, d_xp, st), "rhs copy");
-    DCT_CUDA(dct::run_solve_f64(P, d_xp, k, st, false, copy), "solve launch");
+    DCT_CUDA(dct::run_solve_f64(P, d_xp, k, st, false, copy ? d_bp : nullptr, bstride),
+             "solve launch");
     return DCT_OK;
   }
   return solve_refined(P, d_bp, bstride, k, d_xp, st);

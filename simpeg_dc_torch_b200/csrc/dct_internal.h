@@ -277,6 +277,10 @@ struct dct_plan {
   int64_t stamp = 0;
   const int32_t* d_sn_of = nullptr;   // supernode of each row (permuted order)
   const int32_t* d_parent = nullptr;  // parent supernode, -1: a root
+  // float64 plans whose first forward launch is of single-panel leaves, and
+  // without marks: the rows of all other supernodes
+  const int32_t* d_inner = nullptr;
+  int32_t n_inner = 0;
   int32_t* nz = nullptr;              // nbatch * nsuper marks of a solve (launch_rhs_in)
   const int32_t* d_tc = nullptr;   // f32 plans: supernodes solved by the tensor-core
   int32_t n_tc = 0;                //   products, and how many they are
@@ -336,6 +340,9 @@ struct SolveArgs {
   // reach, nsuper marks per system (null: all of them)
   const int32_t* nz;
   int nsuper;
+  // forward launch of leaves: where their right-hand sides are (null: in A)
+  const T* b;
+  int64_t bstride;
 };
 template <typename T>
 __device__ __forceinline__ bool rhs_reaches(const SolveArgs<T>& g, int s, int b) {
@@ -363,7 +370,8 @@ void set_last_error(const char* msg);
 cudaError_t run_factor(dct_plan* P, const void* vals, int vals_dtype,
                        int64_t vals_stride, cudaStream_t st);
 cudaError_t run_solve_f64(dct_plan* P, double* xa, int k, cudaStream_t st,
-                          bool transposed = false, bool marked = false);
+                          bool transposed = false, const double* b = nullptr,
+                          int64_t bstride = 0);
 cudaError_t run_solve_f32(dct_plan* P, int k, cudaStream_t st, bool marked = false);
 // complex128 plans: the permuted right-hand side in xa (solution left there)
 cudaError_t run_solve_c128(dct_plan* P, cplx* xa, int k, cudaStream_t st);
@@ -379,7 +387,8 @@ cudaError_t launch_convert_any(const void* src, int src_dtype, int64_t sstride,
 // floats in a row of the float32 plans' right-hand sides (see solve.cu)
 inline int rhs_ld(int k) { return (k + 3) & ~3; }
 // b (float64, permuted) -> the right-hand sides of a float32 or float64 solve,
-// marking the supernodes that they reach
+// marking the supernodes that they reach (float64 plans with d_inner: those rows
+// only, the others are read from b)
 cudaError_t launch_rhs_in(dct_plan* P, const double* b, int64_t bstride, int k, void* rhs,
                           cudaStream_t st);
 cudaError_t launch_residual(dct_plan* P, const double* b, int64_t bstride,

@@ -241,20 +241,22 @@ __device__ __forceinline__ void load_quad(const double* p, int left, double (&v)
 // system, the supernodes that a nonzero row belongs to (sn_of) and those above
 // them: the sources of a survey are a few electrodes, and the large forward
 // products of every other supernode have nothing to do.  A walk upwards ends
-// at a mark: whoever set that one walks on from it.
+// at a mark: whoever set that one walks on from it.  rows (null: all n of them):
+// the rows to copy.
 template <typename T, int V>
 __global__ void k_rhs_in(const double* __restrict__ b, int64_t bstride, int n, int k, int kp,
-                         T* __restrict__ rhs, const int32_t* __restrict__ sn_of,
+                         T* __restrict__ rhs, const int32_t* __restrict__ rows, int nrows,
+                         const int32_t* __restrict__ sn_of,
                          const int32_t* __restrict__ parent, int32_t* nz, int nsuper) {
   const int kq = kp / 4 + (kp % 4 != 0);
-  const int64_t total = int64_t(n) * kq;
+  const int64_t total = int64_t(nrows) * kq;
   const double* Bv = b + int64_t(blockIdx.y) * bstride;
   T* R = rhs + int64_t(blockIdx.y) * n * kp;
   volatile int32_t* mark = nz + (nz != nullptr ? int64_t(blockIdx.y) * nsuper : 0);
   for (int64_t idx = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; idx < total;
        idx += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t i = idx / kq;
-    const int j = static_cast<int>(idx - i * kq) * 4, left = k - j;
+    const int64_t q = idx / kq, i = rows != nullptr ? rows[q] : q;
+    const int j = static_cast<int>(idx - q * kq) * 4, left = k - j;
     double v[4];
     load_quad<V>(Bv + i * k + j, left, v);
     T* r = R + i * kp + j;
@@ -487,7 +489,9 @@ cudaError_t launch_tiles(dct_plan* P, int kind, const SolveArgs<T>& g, SmallShap
                          int64_t count, cudaStream_t st) {
   constexpr int V = 16 / sizeof(T);
   sh.wide = g.k % V == 0 && (reinterpret_cast<uintptr_t>(g.A) & 15) == 0 &&
-            (reinterpret_cast<uintptr_t>(g.B) & 15) == 0;
+            (reinterpret_cast<uintptr_t>(g.B) & 15) == 0 &&
+            (g.b == nullptr ||
+             ((reinterpret_cast<uintptr_t>(g.b) & 15) == 0 && g.bstride % V == 0));
   const bool small = kind == kFwdSmall || kind == kBwdSmall;
   switch (small ? small_columns<T>(g.k, sh.w, sh.nb) : tile_columns(g.k)) {
     case 8: return launch_tiles<T, 8>(P, kind, g, sh, count, st);
@@ -507,14 +511,15 @@ inline dim3 grid1d(int64_t total, int ny) {
 // M = U^T, so the forward pass runs on M and the backward pass on L)
 template <typename T>
 cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
-                       bool transposed = false, bool marked = false) {
+                       bool transposed = false, bool marked = false,
+                       const double* b = nullptr, int64_t bstride = 0) {
   cudaError_t e = cudaSuccess;
   SolveArgs<T> g{P->ds, nullptr, static_cast<const T*>(P->fronts), P->front_stride,
                  static_cast<const T*>(P->dinv), P->d_dinv_off, P->dinv_stride,
                  bufA, bufB, P->sym.n, k, 1, P->status,
                  static_cast<const T*>(P->linv), P->d_linv_off, P->linv_stride,
                  P->dtype == DCT_F32 && P->ir != nullptr ? &P->ir->done : nullptr,
-                 marked ? P->nz : nullptr, P->sym.nsuper};
+                 marked ? P->nz : nullptr, P->sym.nsuper, nullptr, 0};
   constexpr bool kTc = sizeof(T) == 4;
   const size_t work = sizeof(T) * size_t(P->nbatch) * P->sym.n * k;
   const double nb = P->nbatch;
@@ -553,6 +558,12 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
           cudaSuccess)
         return e;
       g.tasks = sc->d_tasks + L.first;
+      if constexpr (std::is_same_v<T, double>) {
+        // the first forward launch takes the rows that launch_rhs_in left out
+        const bool here = pass == 0 && li == 0 && b != nullptr && P->d_inner != nullptr;
+        g.b = here ? b : nullptr;
+        g.bstride = bstride;
+      }
       switch (L.kind) {
         case kFwdLinvTc:
         case kFwdBndTc:
@@ -581,11 +592,13 @@ cudaError_t solve_impl(dct_plan* P, T* bufA, T* bufB, int k, cudaStream_t st,
 }  // namespace
 
 // f64 plans: the permuted right-hand side is in `xa` (buffer A) and the
-// solution is left there; P->bufB serves as buffer B.  marked: launch_rhs_in
-// marked the supernodes that its rows reach.
+// solution is left there; P->bufB serves as buffer B.  b (null: all of it is in
+// xa): launch_rhs_in prepared the solve, with the right-hand sides still in b,
+// bstride apart for the systems.
 cudaError_t run_solve_f64(dct_plan* P, double* xa, int k, cudaStream_t st,
-                          bool transposed, bool marked) {
-  return solve_impl<double>(P, xa, static_cast<double*>(P->bufB), k, st, transposed, marked);
+                          bool transposed, const double* b, int64_t bstride) {
+  return solve_impl<double>(P, xa, static_cast<double*>(P->bufB), k, st, transposed,
+                            b != nullptr, b, bstride);
 }
 
 // complex128 plans: as float64, on complex buffers
@@ -684,13 +697,16 @@ cudaError_t launch_rhs_in(dct_plan* P, const double* b, int64_t bstride, int k, 
         cudaMemsetAsync(P->nz, 0, sizeof(int32_t) * size_t(P->nbatch) * nsuper, st);
     if (e != cudaSuccess) return e;
   }
-  const dim3 g = grid1d(int64_t(n) * ((kp + 3) / 4), P->nbatch);
+  const int32_t* rows = f32 ? nullptr : P->d_inner;   // float64: see run_solve_f64
+  const int nrows = rows != nullptr ? P->n_inner : n;
+  if (nrows == 0) return cudaSuccess;
+  const dim3 g = grid1d(int64_t(nrows) * ((kp + 3) / 4), P->nbatch);
   // the copies of the float64 rows are as wide as both sides allow
   const bool even = even_rows(b, bstride, k) &&
                     (f32 || (reinterpret_cast<uintptr_t>(rhs) & 15) == 0);
   auto go = [&](auto* out, auto fn) {
-    fn<<<g, kThreads, 0, st>>>(b, bstride, n, k, kp, out, P->d_sn_of, P->d_parent, P->nz,
-                               nsuper);
+    fn<<<g, kThreads, 0, st>>>(b, bstride, n, k, kp, out, rows, nrows, P->d_sn_of, P->d_parent,
+                               P->nz, nsuper);
   };
   if (f32)
     go(static_cast<float*>(rhs), even ? k_rhs_in<float, 2> : k_rhs_in<float, 1>);

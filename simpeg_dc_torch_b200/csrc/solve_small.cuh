@@ -523,8 +523,9 @@ k_fwd_small(SolveArgs<T> g, SmallShape sh) {
   T* A = g.A + int64_t(b) * g.n * g.k;
   T* Bo = g.B + int64_t(b) * g.n * g.k;
   const bool wide = sh.wide != 0;
+  const T* src = g.b != nullptr ? g.b + b * g.bstride : A;
   auto load_b = [&](int j0) {
-    small_load_rhs<T, NC>(Xt, A, g.k, j0, min(NC, je - j0), w, wide,
+    small_load_rhs<T, NC>(Xt, src, g.k, j0, min(NC, je - j0), w, wide,
                           [&](int r) { return first + r; });
   };
   for (int i = threadIdx.x; i < min(kSmallRows, N - w); i += kThreads) rows_s[i] = rows[w + i];
