@@ -387,16 +387,23 @@ def count_launches(eng):
     sym = eng.solver._sym
     code = eng.solver._code
     nl = {}
-    for which in range(5):
+    for which in (1, 2, 4):
         _, launches = sym.schedule(code, which)
         nl[which] = int((launches[:, 3] > 0).sum())
-    # factor: schedule + panel inverses + supernode inverses, the lower-
-    # triangle clearing launched with every large-front scatter, and the
-    # float64 value copy of float32 plans
-    _, fl = sym.schedule(code, 0)
-    nscatter = int(((fl[:, 0] == 1) & (fl[:, 3] > 0)).sum())
-    factor = nl[0] + nscatter + nl[3] + nl[4] + (1 if code == 1 else 0)
+    # factor: schedule + supernode inverses, the assembly launched with every
+    # large-front scatter (which leaves the extend-add of children beyond the
+    # second), and the float64 value copy of float32 plans
+    _, fl = sym.schedule(code, 0 if code == 1 else 5)
+    fl = fl[fl[:, 3] > 0]
+    nscatter = int((fl[:, 0] == 1).sum())
+    assembled = int(((fl[:, 0] == 2) & (fl[:, 4] < 2)).sum())
+    factor = len(fl) - assembled + nscatter + nl[4] + (1 if code == 1 else 0)
     passes = nl[1] + nl[2]
+    # float32 plans with one-CTA and tensor-core supernodes clear the rows of the
+    # latter before each pass
+    tc = sym.schedule(code, 1)[1][:, 0] >= 15
+    if code == 1 and tc.any() and not tc.all():
+        passes += 2
     if code == 0:
         solve = 1 + passes                       # rhs copy + substitution
     else:

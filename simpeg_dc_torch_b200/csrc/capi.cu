@@ -274,7 +274,7 @@ void account_solve(const dct::Symbolic& S, dct::Schedule* sc, double es) {
   }
 }
 
-// trailing-update tile: 64 for float64 (CUDA cores), 128 for float32
+// trailing-update tile: 64 for float64, 128 for float32
 // (tcgen05 tensor-core tiles, M = N = 128)
 int update_tile(int dtype) { return dtype == DCT_F32 ? 128 : dct::kUpdateTile; }
 

@@ -2,9 +2,9 @@
 // permuted order, on row-major (n, k) right-hand sides.
 //
 // Per tree level (forward bottom-up, backward top-down):
-//   supernodes of one panel (ns <= 64): one CTA per (supernode, system, up to
-//     64 right-hand sides) does the whole step with the stored panel inverse
-//     D^{-1} (solve_small.cuh);
+//   supernodes of one panel (ns <= 64): one CTA per supernode, system and one
+//     or more chunks of up to 64 right-hand sides does the whole step with the
+//     stored panel inverse D^{-1} (solve_small.cuh);
 //   larger supernodes: products with the explicit supernode inverse
 //     L_ss^{-1} (formed after the factorization) and with the boundary block
 //     L_Bs, in 64-row tiles (float64 on the double tensor cores, complex on the
