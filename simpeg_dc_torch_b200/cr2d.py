@@ -32,10 +32,14 @@ from .solver import _stream_ptr, make_batch_solver, sparse_solve_batch
 
 
 class _Values(torch.autograd.Function):
-    """L x for the assembly map L of a fused path (float64)."""
+    """L x for the assembly map L of a fused path (float64).  The kernels read the path's nC
+    entries of x by its address, so its length is checked here, before any launch."""
 
     @staticmethod
     def forward(ctx, x, path):
+        if x.dim() != 1 or x.numel() != path.nC:
+            raise ValueError(f"expected one value for each of {path.nC} cells, got shape "
+                             f"{tuple(x.shape)}")
         ctx.path = path
         x = x.contiguous()
         y = torch.empty(path.nbatch * path.nnzA, dtype=torch.float64, device=x.device)

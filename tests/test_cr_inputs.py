@@ -1,0 +1,46 @@
+"""TorchCR2D's products with the assembly map, without a GPU: the two kernels are stood in for by
+recorders, so what is checked is what reaches them."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from simpeg_dc_torch_b200 import cr2d
+
+NC, NNZ, NKY = 6, 9, 2
+
+
+class Kernels:
+    """Records the calls; every output stays as it was allocated."""
+
+    def __init__(self):
+        self.calls = []
+
+    def dct_csr_spmv(self, *args):
+        self.calls.append("dct_csr_spmv")
+        return 0
+
+    def dct_values_vjp(self, *args):
+        self.calls.append("dct_values_vjp")
+        return 0
+
+
+@pytest.fixture
+def kernels(monkeypatch):
+    k = Kernels()
+    monkeypatch.setattr(cr2d.nat, "lib", lambda: k)
+    monkeypatch.setattr(cr2d, "_stream_ptr", lambda device: 0)
+    return k
+
+
+def path():
+    t = torch.zeros(1)
+    return SimpleNamespace(nC=NC, nnzA=NNZ, nbatch=NKY, L_ptr=t, L_col=t, L_val=t, Lt_ptr=t,
+                           Lt_col=t, Lt_val=t)
+
+
+@pytest.mark.parametrize("n", [0, 1, NC - 1, NC + 1, 2 * NC])
+def test_wrong_length_is_refused_before_any_launch(kernels, n):
+    with pytest.raises(ValueError, match=f"{NC} cells"):
+        cr2d._Values.apply(torch.zeros(n, dtype=torch.float64), path())
+    assert kernels.calls == []
