@@ -33,7 +33,8 @@ from .solver import _stream_ptr, make_batch_solver, sparse_solve_batch
 
 class _Values(torch.autograd.Function):
     """L x for the assembly map L of a fused path (float64).  The kernels read the path's nC
-    entries of x by its address, so its length is checked here, before any launch."""
+    entries of x by its address, so its length is checked here, before any launch, and they run on
+    the current device, which is made the tensors' own."""
 
     @staticmethod
     def forward(ctx, x, path):
@@ -43,9 +44,10 @@ class _Values(torch.autograd.Function):
         ctx.path = path
         x = x.contiguous()
         y = torch.empty(path.nbatch * path.nnzA, dtype=torch.float64, device=x.device)
-        nat.check(nat.lib().dct_csr_spmv(
-            y.numel(), path.L_ptr.data_ptr(), path.L_col.data_ptr(), path.L_val.data_ptr(),
-            x.data_ptr(), y.data_ptr(), _stream_ptr(x.device)), "dct_csr_spmv")
+        with torch.cuda.device(x.device):
+            nat.check(nat.lib().dct_csr_spmv(
+                y.numel(), path.L_ptr.data_ptr(), path.L_col.data_ptr(), path.L_val.data_ptr(),
+                x.data_ptr(), y.data_ptr(), _stream_ptr(x.device)), "dct_csr_spmv")
         return y
 
     @staticmethod
@@ -53,10 +55,11 @@ class _Values(torch.autograd.Function):
         path, gy = ctx.path, gy.contiguous()
         minus = torch.full((path.nC,), -1.0, dtype=torch.float64, device=gy.device)
         gx = torch.empty_like(minus)
-        nat.check(nat.lib().dct_values_vjp(   # -sigma * (L^T g) at sigma = -1
-            path.nC, path.Lt_ptr.data_ptr(), path.Lt_col.data_ptr(), path.Lt_val.data_ptr(),
-            minus.data_ptr(), gy.data_ptr(), gx.data_ptr(), _stream_ptr(gy.device)),
-            "dct_values_vjp")
+        with torch.cuda.device(gy.device):
+            nat.check(nat.lib().dct_values_vjp(   # -sigma * (L^T g) at sigma = -1
+                path.nC, path.Lt_ptr.data_ptr(), path.Lt_col.data_ptr(), path.Lt_val.data_ptr(),
+                minus.data_ptr(), gy.data_ptr(), gx.data_ptr(), _stream_ptr(gy.device)),
+                "dct_values_vjp")
         return gx, None
 
 
