@@ -25,6 +25,7 @@ the map on every call and formed the data of every source at every receiver
 from __future__ import annotations
 
 import torch
+from torch.autograd.function import once_differentiable
 
 from . import _native as nat
 from .simulation2d import TorchDC2D
@@ -34,7 +35,8 @@ from .solver import _stream_ptr, make_batch_solver, sparse_solve_batch
 class _Values(torch.autograd.Function):
     """L x for the assembly map L of a fused path (float64).  The kernels read the path's nC
     entries of x by its address, so its length is checked here, before any launch, and they run on
-    the current device, which is made the tensors' own."""
+    the current device, which is made the tensors' own.  First order only, like the solve that
+    follows it: the backward is a kernel that autograd does not see."""
 
     @staticmethod
     def forward(ctx, x, path):
@@ -51,6 +53,7 @@ class _Values(torch.autograd.Function):
         return y
 
     @staticmethod
+    @once_differentiable
     def backward(ctx, gy):
         path, gy = ctx.path, gy.contiguous()
         minus = torch.full((path.nC,), -1.0, dtype=torch.float64, device=gy.device)

@@ -60,3 +60,11 @@ def test_kernels_run_on_the_tensors_device(kernels):
     cr2d._Values.apply(x, path()).sum().backward()
     assert kernels.calls == [("dct_csr_spmv", x.device), ("dct_values_vjp", x.device)]
     assert kernels.current is None
+
+
+def test_second_order_is_refused(kernels):
+    x = torch.zeros(NC, dtype=torch.float64, requires_grad=True)
+    gy = torch.ones(NKY * NNZ, dtype=torch.float64, requires_grad=True)
+    (gx,) = torch.autograd.grad(cr2d._Values.apply(x, path()), x, gy, create_graph=True)
+    with pytest.raises(RuntimeError, match="once_differentiable"):
+        gx.sum().backward()

@@ -32,3 +32,13 @@ def test_one_chargeability_for_all_cells(engine):
     ref = eng.voltages(m, torch.full_like(m, one.item()))   # (0.1 as a float32)
     eng.check()
     assert float((V - ref).abs().max()) <= 1e-12 * float(ref.abs().max())
+
+
+def test_first_order_gradient_under_create_graph(engine):
+    eng, m = engine
+    x = torch.cat([m, torch.full_like(m, 0.1)]).requires_grad_(True)
+    phi = lambda: sum((d ** 2).sum() for d in eng.dpred(x))  # noqa: E731
+    (ref,) = torch.autograd.grad(phi(), x)
+    (g,) = torch.autograd.grad(phi(), x, create_graph=True)
+    eng.check()
+    assert float((g - ref).detach().abs().max()) <= 1e-12 * float(ref.abs().max())
