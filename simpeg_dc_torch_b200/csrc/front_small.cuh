@@ -58,34 +58,13 @@ __host__ __device__ constexpr size_t small_smem(int N) {
 // twice as many of them share an SM and hide one another's pivot chains.
 constexpr int kSmallNarrow = 112;
 
-// d = sqrt(p), r = 1 / d of a pivot.  Double: the exponent is halved apart,
-// so that the float estimate y0 of the reciprocal root works on a number m in
-// [1, 4) whatever the scale of the matrix; with t = 1 - m y0^2 (about 2^-22)
-// one step of third order, y0 (1 + t/2 + 3 t^2/8), leaves t^3, below the
-// rounding, in fewer dependent operations than Newton-Raphson steps would
-// take; the root itself gets one correction.
+// d = sqrt(p), r = 1 / d of a pivot, both correctly rounded in float and double
+// at any scale.  All pivots of a block take theirs at once, one per lane, off
+// the chain from pivot to pivot.
 template <typename T>
 __device__ __forceinline__ void pivot_root(T p, T& d, T& r) {
   d = sqrt(p);
   r = T(1) / d;
-}
-template <>
-__device__ __forceinline__ void pivot_root<double>(double p, double& d, double& r) {
-  const int hi = __double2hiint(p);
-  const int e = ((hi >> 20) - 1023) & ~1;
-  if (hi < (1 << 20)) {   // subnormal
-    d = sqrt(p);
-    r = 1.0 / d;
-    return;
-  }
-  const double m = __hiloint2double(hi - e * (1 << 20), __double2loint(p));   // in [1, 4)
-  const double y0 = double(rsqrtf(float(m)));
-  const double t = fma(-m * y0, y0, 1.0);
-  const double y = fma(t * y0, fma(0.375, t, 0.5), y0);
-  double q = m * y;
-  q = fma(0.5 * y, fma(-q, q, m), q);
-  r = __hiloint2double(__double2hiint(y) - e / 2 * (1 << 20), __double2loint(y));
-  d = __hiloint2double(__double2hiint(q) + e / 2 * (1 << 20), __double2loint(q));
 }
 
 // entry (r, c) of the panel inverse kept transposed above the diagonal
