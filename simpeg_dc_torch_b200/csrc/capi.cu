@@ -1006,14 +1006,15 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
   // forward products (the single-panel ones look at their own rows), so plans
   // that spend less than half of the forward pass there go without: in 2-D
   // grids the marks cost as much as they save (56 us a solve against 27 without
-  // and 20 us of products, line of 38 sources)
+  // and 20 us of products, line of 38 sources).  General plans alike: their
+  // forward pass runs the same launches on L
   double large = 0, all = 0;
   for (size_t i = 0; i < P->fwd.launches.size(); ++i) {
     all += P->fwd.flops[i];
     if (P->fwd.launches[i].kind != dct::kFwdSmall) large += P->fwd.flops[i];
   }
   const bool marks = large >= 0.5 * all && large > 0;
-  if (marks && dtype != DCT_C128 && !P->lu) {
+  if (marks && dtype != DCT_C128) {
     std::vector<int32_t> sn_of(S.n);
     for (int s = 0; s < S.nsuper; ++s)
       for (int i = S.sn_first[s]; i < S.sn_first[s + 1]; ++i) sn_of[i] = s;
