@@ -81,10 +81,11 @@ int dct_symbolic_get_array(const dct_symbolic* sym, const char* name,
                            int64_t* size_bytes);
 
 /* Host-side copy of the launch schedule a plan of this dtype would run
- * (which: 0 factorization, 1 forward, 2 backward substitution, 3 panel
- * inverses, 4 supernode inverses, 5 factorization with the trailing updates
- * in blocks of four panels, as float64 and complex plans run it -- 0 gives
- * their update after every panel), for
+ * (which: 0 factorization -- for float64 and complex with an update after every
+ * panel, which no plan runs: the reference of the replays --, 1 forward, 2
+ * backward substitution, 3 inverses of the single-CTA fronts' panels, which
+ * general plans run, 4 supernode inverses, 5 factorization with the trailing
+ * updates in the blocks of dct_tuning_default), for
  * inspection and CPU-side replay in tests.  tasks: 4 int32 per task
  * (supernode, panel or K start, t0, t1 or K end); launches: 5 int64 per launch (kind, level,
  * first task, task count, arg).  With null outputs only the counts are set. */
@@ -113,11 +114,12 @@ int dct_plan_create(const dct_symbolic* sym, int32_t nbatch, int32_t max_rhs,
  *   small_front_max   largest front factored by one CTA in shared memory
  *                     (32 .. 224 float32, 32 .. 160 float64); larger fronts
  *                     take the panel / trailing-update path
- *   update_block      panels per block of the float32 trailing update (1..4;
- *                     the deferred update after a block has K = 64 x this)
+ *   update_block      panels per block of the trailing update (the deferred
+ *                     update after a block has K = 64 x this): 1..4 in float32
+ *                     plans, 4 in float64 and complex ones
  *   solve_target      float32 substitution: fewest tasks a launch is split
  *                     into (K ranges halved until reached)
- *   solve_split_max   float32 substitution: longest K piece of one task
+ *   solve_split_max   float32 substitution: longest K piece of one task (16 .. 1024)
  *   solve_split_min   float32 substitution: shortest K piece
  *   small_tc          single-panel supernodes on the tensor-core products:
  *                     1 yes, 2 no (CUDA-core one-CTA kernels), <= 0 decided

@@ -181,7 +181,9 @@ int small_front_limit(int dtype) {
 dct_tuning default_tuning(int dtype) {
   dct_tuning t;
   t.small_front_max = small_front_limit(dtype);
-  t.update_block = dtype == DCT_F32 ? dct::kUpdateBlockPanels : 1;
+  // float64 and complex: a tile is read and written once per 256 columns instead
+  // of once per 64
+  t.update_block = dtype == DCT_F32 ? dct::kUpdateBlockPanels : dct::kUpdateBlockWide;
   t.solve_target = kTcTargetCtas;
   t.solve_split_max = kTcSplitK;
   t.solve_split_min = kTcSplitMin;
@@ -194,7 +196,7 @@ dct_tuning resolve_tuning(int dtype, const dct_tuning* in) {
   if (in == nullptr) return t;
   const int smax = small_front_limit(dtype);
   if (in->small_front_max > 0) t.small_front_max = std::max(32, std::min(smax, in->small_front_max));
-  // float64 fronts update after every panel (no blocking)
+  // float64 and complex plans keep their default
   if (in->update_block > 0 && dtype == DCT_F32) t.update_block = std::min(4, in->update_block);
   if (in->solve_target > 0) t.solve_target = in->solve_target;
   if (in->solve_split_max > 0)
@@ -203,15 +205,6 @@ dct_tuning resolve_tuning(int dtype, const dct_tuning* in) {
   t.solve_split_min = std::min(t.solve_split_min, t.solve_split_max);
   if (in->small_tc > 0) t.small_tc = std::min(2, in->small_tc);
   return t;
-}
-
-
-// Panels per block of a plan's trailing update.  Float64 and complex plans
-// take blocks of kUpdateBlockWide panels whatever the tuning says (it tunes
-// the float32 blocks): a tile is then read and written once per 256 columns
-// instead of once per 64.
-int plan_update_block(int dtype, const dct_tuning& t) {
-  return dtype == DCT_F32 ? t.update_block : dct::kUpdateBlockWide;
 }
 
 void account_solve(const dct::Symbolic& S, dct::Schedule* sc, double es) {
@@ -818,8 +811,7 @@ int dct_symbolic_get_schedule(const dct_symbolic* h, int32_t dtype, int32_t whic
   const dct_tuning tu = default_tuning(dtype);
   const int small_max = tu.small_front_max;
   build_factor_schedule(h->sym, small_max, update_tile(dtype),
-                        which == 5 ? plan_update_block(dtype, tu) : tu.update_block,
-                        dtype == DCT_F32, &f);
+                        which == 0 && dtype != DCT_F32 ? 1 : tu.update_block, dtype == DCT_F32, &f);
   build_solve_schedules(h->sym, dtype, tu, &fw, &bw);
   std::vector<int64_t> off;
   int64_t tot = 0;
@@ -934,7 +926,7 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
   }
   P->tune = resolve_tuning(dtype, tuning);
   const int small_max = P->tune.small_front_max;
-  P->update_bpan = plan_update_block(dtype, P->tune);
+  P->update_bpan = P->tune.update_block;
   build_factor_schedule(S, small_max, update_tile(dtype), P->update_bpan, dtype == DCT_F32,
                         &P->fact);
   {
