@@ -86,7 +86,9 @@ int dct_symbolic_get_array(const dct_symbolic* sym, const char* name,
  * backward substitution, 3 inverses of the single-CTA fronts' panels, which
  * general plans run, 4 supernode inverses, 5 factorization with the trailing
  * updates in the blocks of dct_tuning_default), for
- * inspection and CPU-side replay in tests.  tasks: 4 int32 per task
+ * inspection and CPU-side replay in tests.  A plan's factorization takes the
+ * first two children of a large front with its scatter, where these schedules
+ * have an extend-add launch for each child.  tasks: 4 int32 per task
  * (supernode, panel or K start, t0, t1 or K end); launches: 5 int64 per launch (kind, level,
  * first task, task count, arg).  With null outputs only the counts are set. */
 int dct_symbolic_get_schedule(const dct_symbolic* sym, int32_t dtype,

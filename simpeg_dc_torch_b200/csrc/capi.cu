@@ -91,9 +91,20 @@ void account_factor(const dct::Symbolic& S, dct::Schedule* sc, double es,
           b += es * (double(N) * N + upd) + nent * (es + 8);
           break;
         }
-        case dct::kLargeScatter:
-          b += double(S.amap_ptr[s + 1] - S.amap_ptr[s]) * (2 * es + 8);
+        case dct::kLargeScatter: {
+          // with the assembly: the triangle written, the first two children's
+          // update matrices read (and the second's added to the first's)
+          const double nent = double(S.amap_ptr[s + 1] - S.amap_ptr[s]);
+          double el = double(N) * (N + 1) / 2;
+          for (int u = 0; u < 2 && S.child_ptr[s] + u < S.child_ptr[s + 1]; ++u) {
+            const double nbc = S.nb(S.child[S.child_ptr[s] + u]);
+            el += nbc * (nbc + 1) / 2;
+            if (u == 1) f += nbc * (nbc + 1) / 2;
+          }
+          f += nent;
+          b += el * es + nent * (3 * es + 8);
           break;
+        }
         case dct::kLargeExtendAdd: {
           const int nbc = S.nb(t.t0);
           double cols = std::min(8, nbc - t.t1), el = 0;
@@ -276,8 +287,11 @@ int update_tile(int dtype) { return dtype == DCT_F32 ? 128 : dct::kUpdateTile; }
 #endif
 constexpr int kSmallBucketMin = 256;   // fronts: about two CTAs per SM of a B200
 
+// slot0: the first child that gets extend-add launches.  A plan's assembly takes
+// the first two with the scatter (k_large_assemble); the exported schedules add
+// every child.
 void build_factor_schedule(const dct::Symbolic& S, int small_max, int utile, int bpan,
-                           bool align8, dct::Schedule* out) {
+                           bool align8, int slot0, dct::Schedule* out) {
   auto& T = out->tasks;
   auto& L = out->launches;
   for (int lv = 0; lv < S.nlevels; ++lv) {
@@ -326,7 +340,7 @@ void build_factor_schedule(const dct::Symbolic& S, int small_max, int utile, int
     int max_children = 0;
     for (int s : large)
       max_children = std::max(max_children, S.child_ptr[s + 1] - S.child_ptr[s]);
-    for (int slot = 0; slot < max_children; ++slot) {
+    for (int slot = slot0; slot < max_children; ++slot) {
       Launch l{dct::kLargeExtendAdd, lv, int64_t(T.size()), 0, slot};
       for (int s : large) {
         int nch = S.child_ptr[s + 1] - S.child_ptr[s];
@@ -811,7 +825,8 @@ int dct_symbolic_get_schedule(const dct_symbolic* h, int32_t dtype, int32_t whic
   const dct_tuning tu = default_tuning(dtype);
   const int small_max = tu.small_front_max;
   build_factor_schedule(h->sym, small_max, update_tile(dtype),
-                        which == 0 && dtype != DCT_F32 ? 1 : tu.update_block, dtype == DCT_F32, &f);
+                        which == 0 && dtype != DCT_F32 ? 1 : tu.update_block, dtype == DCT_F32, 0,
+                        &f);
   build_solve_schedules(h->sym, dtype, tu, &fw, &bw);
   std::vector<int64_t> off;
   int64_t tot = 0;
@@ -927,7 +942,7 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
   P->tune = resolve_tuning(dtype, tuning);
   const int small_max = P->tune.small_front_max;
   P->update_bpan = P->tune.update_block;
-  build_factor_schedule(S, small_max, update_tile(dtype), P->update_bpan, dtype == DCT_F32,
+  build_factor_schedule(S, small_max, update_tile(dtype), P->update_bpan, dtype == DCT_F32, 2,
                         &P->fact);
   {
     int sms = 0;

@@ -543,7 +543,6 @@ cudaError_t factor_impl(dct_plan* P, const void* vals, int vals_dtype,
             P->d_tr);
         break;
       case kLargeExtendAdd:
-        if (L.arg < 2) break;   // the first two children: k_large_assemble
         for (T* buf : {fronts, fronts2}) {
           if (buf == nullptr) continue;
           k_large_extend_add<T><<<grid, kThreads, 0, st>>>(P->ds, t, buf, P->front_stride);
