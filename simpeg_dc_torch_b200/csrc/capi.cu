@@ -1049,8 +1049,7 @@ int dct_plan_create_tuned(const dct_symbolic* h, int32_t nbatch, int32_t max_rhs
     if ((rc = upload(P, inner, &P->d_inner))) return bail(rc);
   }
   if ((rc = upload_schedule(P, &P->fact)) || (rc = upload_schedule(P, &P->fwd)) ||
-      (rc = upload_schedule(P, &P->bwd)) || (rc = upload_schedule(P, &P->inv)) ||
-      (rc = upload_schedule(P, &P->linv_sched)))
+      (rc = upload_schedule(P, &P->bwd)) || (rc = upload_schedule(P, &P->linv_sched)))
     return bail(rc);
   const size_t es = esize(dtype);
   P->front_stride = S.front_total;
@@ -1124,6 +1123,7 @@ int dct_plan_create_general(const dct_symbolic* h, int32_t nbatch, int32_t max_r
   const int32_t* d_tr = nullptr;
   if ((rc = upload(P, tr, &d_tr))) return bail(rc);
   P->d_tr = d_tr;
+  if ((rc = upload_schedule(P, &P->inv))) return bail(rc);
   if ((rc = alloc(P, 8 * size_t(P->sym.front_total) * nbatch, &P->fronts2, "front storage (U^T)")))
     return bail(rc);
   if ((rc = alloc(P, 8 * size_t(P->dinv_stride) * nbatch, &P->dinv2, "panel inverses (U^T)")))

@@ -257,7 +257,8 @@ struct dct_plan {
   std::vector<int64_t> asm_first, asm_count;
   dct::Schedule fwd;               // forward substitution schedule
   dct::Schedule bwd;               // backward substitution schedule
-  dct::Schedule inv;               // diagonal-block inverses (one launch)
+  dct::Schedule inv;               // general plans: inverses of the single-CTA
+                                   // fronts' diagonal blocks (one launch)
   void* dinv = nullptr;            // nbatch * dinv_stride elements of dtype
   int64_t dinv_stride = 0;         // per system: sum over panels of w^2
   const int64_t* d_dinv_off = nullptr;   // per supernode, first panel inverse
