@@ -19,8 +19,9 @@
 //   backward: y_s -= L_Bs^T x_B with x_B (rows of ancestors, final) in A;
 //             x_s = L_ss^{-T} y_s goes to A.
 // The tensor-core kinds split long K ranges over CTAs and accumulate with
-// atomics, so in float32 plans B is cleared before the forward pass and A
-// (whose right-hand side is consumed by then) before the backward pass.
+// atomics, so in float32 plans the rows of the supernodes that take them are
+// cleared in B before the forward pass and in A (whose right-hand side is
+// consumed by then) before the backward pass.
 #include <cuda_runtime.h>
 
 #include <algorithm>
